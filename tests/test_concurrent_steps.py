@@ -1,0 +1,60 @@
+"""Repeated steps: from the 33rd launch on, a step runs as a graph that holds only the orders
+its data needs.  Its memory must equal, word for word, that of the same steps played op by op
+in tape order."""
+import numpy as np
+import pytest
+
+from tests import helpers
+from thunderengine_web_b200 import scenario, timestep
+
+STEPS = 36   # four of them past the chain
+
+
+def _both(tape, init, mode):
+    out = []
+    for graph in (True, False):
+        r = helpers.gpu_replayer(tape, init, hashes=False, mode=mode if graph else 0)
+        if graph:
+            r.encode_steps(STEPS)
+        else:
+            for _ in range(STEPS):
+                r.run_ops(0, r.num_ops - 1)
+        out.append(r.read(r.buffers_end))
+        base = list(r.base)
+        r.close()
+    return out, base
+
+
+# 12x10x8: the smallest; 37x29x13: odd extents; 40x24x16 dry on aligned rows
+@pytest.mark.gpu
+@pytest.mark.parametrize('mode', [0, 1])
+@pytest.mark.parametrize('dims,moist,align', [((12, 10, 8), True, False), ((37, 29, 13), True, False),
+                                              ((40, 24, 16), False, True)])
+def test_synthetic_steps_equal_the_ops_in_tape_order(dims, moist, align, mode):
+    run = timestep.Run(scenario.tiny(*dims, dx=500.0, dz=250.0, dt=3.0, nsound=8, us=25.0, align_rows=align), moist=moist)
+    tape = run.tape(1)
+    (graph, ops), base = _both(tape, run.initial_buffers(), mode)
+    if mode == 0:
+        assert np.array_equal(graph, ops)
+        return
+    for name in run.fields:   # fused mode does not keep the step's scratch fields
+        if name not in helpers.SCRATCH:
+            a, b = (helpers.field_view(m, run, base[run.rec.ids['arena']], name) for m in (graph, ops))
+            assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), name
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('mode', [0, 1])
+@pytest.mark.parametrize('name', ['single_cell', 'squall_line'])
+def test_recorded_physics_steps_equal_the_ops_in_tape_order(name, mode):
+    tape, init, _, _ = helpers.load_golden_scenario(name)
+    (graph, ops), base = _both(tape, init, mode)
+    if mode == 0:
+        assert np.array_equal(graph, ops)
+        return
+    arena = next(b['id'] for b in tape['buffers'] if b['arena'])
+    scratch = set(helpers.SCRATCH)
+    for field in tape['fields']:
+        if field not in scratch:
+            a, b = (helpers.field_view(m, tape, base[arena], field) for m in (graph, ops))
+            assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), field

@@ -133,7 +133,7 @@ int te_ensemble_create(te_ctx* const* members, int n, te_ensemble** out) {
     ECU(cudaGraphCreate(&root, 0));
     try {
       for (te_ctx* c : E->members) {
-        cudaGraph_t g = c->plan.capture_step();
+        cudaGraph_t g = c->plan.capture_step(false);  // the members already run side by side
         cudaGraphNode_t node;
         const cudaError_t e = cudaGraphAddChildGraphNode(&node, root, nullptr, 0, g);
         cudaGraphDestroy(g);

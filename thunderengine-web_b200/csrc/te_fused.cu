@@ -1203,8 +1203,72 @@ void FusedStep::build(Plan& P, std::vector<Op>& ops) {
   }
 }
 
-void FusedStep::launch(Plan& P, std::vector<Op>& ops) {
-  for (int q = 0; q < (int)segs.size(); q++) launch_segment(P, ops, q, -1);
+// The words each kernel of a fused phase reads and writes (the phase's scratch fields that
+// the fused kernels do not touch left out).
+static std::vector<Access> halo_accesses(const Plan& P, const HaloArgs& H) {
+  std::vector<Access> acc;
+  for (int q = 0; q < H.nf; q++) acc.push_back(P.access(H.f[q], true));
+  if (H.acc_rrw) acc.push_back(P.access(H.acc_rrw, true));
+  return acc;
+}
+
+static std::vector<Access> adv_accesses(const Plan& P, const AdvArgs& A, int kind) {
+  std::vector<Access> acc;
+  const FluxNames* fs = nullptr;
+  for (auto& c : kFluxSets)
+    if (c.kind == kind) fs = &c;
+  for (int b = 0; b < kMaxBind; b++) {
+    if (b != fs->out_h && A.fx.p[b]) acc.push_back(P.access(A.fx.p[b], false));
+    if (b != fs->out_h && A.fy.p[b]) acc.push_back(P.access(A.fy.p[b], false));
+    if (b != fs->out_z && A.fz.p[b]) acc.push_back(P.access(A.fz.p[b], false));
+    if (b != 3 && b != 4 && b != 5 && b != 11 && b != 19 && A.as.p[b]) acc.push_back(P.access(A.as.p[b], false));
+  }
+  for (const float* f : {A.div3d, A.thterm, A.phiA})
+    if (f) acc.push_back(P.access(f, false));
+  // an RK update that keeps its tendency to itself still reads it on open u, v edges
+  acc.push_back(P.access(A.dest, A.accumulate || A.write_dest));
+  for (float* f : {A.phi, A.fxo, A.fyo, A.fzo})
+    if (f) acc.push_back(P.access(f, true));
+  return acc;
+}
+
+static std::vector<Access> acu_accesses(const Plan& P, const AcuArgs& A, int part) {
+  std::vector<Access> acc;
+  auto add = [&](std::initializer_list<const float*> fields, bool write) {
+    for (const float* f : fields)
+      if (f) acc.push_back(P.access(f, write));
+  };
+  if (part == 0) {
+    add({A.ppd, A.thv, A.uten, A.vten, A.hm}, false);
+    add({A.u, A.v, A.rru, A.rrv}, true);
+  } else if (part == 1) {
+    add({A.u, A.v, A.piadv, A.ppten, A.ppterm, A.pk1, A.pk2, A.qk, A.mm, A.wten, A.hm}, false);
+    add({A.w, A.pp3d, A.ppdw, A.rrw}, true);
+    if (A.saveX) add({A.ppx}, true);
+  } else {
+    add({A.ppdw, A.u, A.v, A.w, A.rrw}, true);
+  }
+  return acc;
+}
+
+void FusedStep::launch(Plan& P, std::vector<Op>& ops, StepDeps* deps) {
+  const FusedData& D = *static_cast<FusedData*>(data);
+  if (!deps) {
+    for (int q = 0; q < (int)segs.size(); q++) launch_segment(P, ops, q, -1);
+    return;
+  }
+  auto run = [&](const std::vector<Access>& acc, int q, int part) {
+    if (deps->run(acc, [&] { launch_segment(P, ops, q, part); }) != cudaSuccess)
+      throw std::runtime_error("capture of a fused segment failed");
+  };
+  for (int q = 0; q < (int)segs.size(); q++) {
+    const FusedSegment& s = segs[q];
+    if (s.kind == kExact) P.launch_exact(ops, s.first, s.last, false, deps);
+    else if (s.kind == kHalo) run(halo_accesses(P, D.halo[s.aux[0]]), q, -1);
+    else if (s.kind == kAdvect) run(adv_accesses(P, D.adv[s.aux[0]], s.aux[1]), q, -1);
+    else
+      for (int part = 0; part < 3; part++) run(acu_accesses(P, D.acu[s.aux[0]], part), q, part);
+  }
 }
 
 void FusedStep::launch_segment(Plan& P, std::vector<Op>& ops, int seg, int part) {

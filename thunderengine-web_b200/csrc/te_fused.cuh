@@ -10,6 +10,7 @@ namespace te {
 
 struct Op;
 struct Plan;
+class StepDeps;
 
 // A step's op list rewritten into segments: runs of exact per-dispatch kernels and
 // fused phase kernels that produce bit-identical prognostic fields.
@@ -23,7 +24,8 @@ struct FusedStep {
   std::vector<FusedSegment> segs;
   void* data = nullptr;  // kernel arguments of the fused segments
   void build(Plan& P, std::vector<Op>& ops);
-  void launch(Plan& P, std::vector<Op>& ops);
+  // the whole step; with deps (during a capture) each kernel after those it depends on only
+  void launch(Plan& P, std::vector<Op>& ops, StepDeps* deps);
   // one segment; part = -1 for all of its kernels, else the index of one of them
   void launch_segment(Plan& P, std::vector<Op>& ops, int seg, int part);
   int launches_per_step() const;

@@ -7,6 +7,7 @@
 #include <string>
 #include <vector>
 
+#include "te_deps.hpp"
 #include "te_fused.cuh"
 #include "te_json.hpp"
 #include "te_kernels.cuh"
@@ -78,6 +79,9 @@ struct Plan {
   uint32_t* M = nullptr;
   uint32_t* H = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
+  cudaGraphExec_t graph_chain = nullptr;  // the chain a concurrent graph_exec replaced, which may still run
+  int graph_runs = 0;             // steps launched since the step, mode or parameters last changed
+  bool graph_concurrent = false;  // graph_exec holds the data's orders only, not the whole chain
   FusedStep fused;
   bool fused_dirty = true;
   AdjointState* adjoint = nullptr;  // checkpoints, undo log and adjoint memory of te_adjoint_*
@@ -88,9 +92,14 @@ struct Plan {
   std::vector<Op> build_ops(const JValue& cmds, const std::map<int, uint64_t>& offs, bool hashes);
   void plan(const char* tj, size_t tl, bool with_hashes);
   void finalize_args(std::vector<Op>& ops);
-  void launch_exact(std::vector<Op>& ops, int first, int last, bool hashes);
+  // with `deps` (during a capture) each op waits only for the ops it depends on
+  void launch_exact(std::vector<Op>& ops, int first, int last, bool hashes, StepDeps* deps = nullptr);
+  Access access(const void* p, bool write) const;         // the tape region a field pointer names
+  std::vector<Access> accesses(const Op& o) const;        // the words one op reads and writes
   void launch_step_graph();
-  cudaGraph_t capture_step();  // the active step (current mode) as a graph, not instantiated
+  // the active step (current mode) as a graph, not instantiated: a chain of its launches in
+  // tape order or, concurrent, with the orders their data needs (te_deps.hpp)
+  cudaGraph_t capture_step(bool concurrent);
   void invalidate_graphs();
   void release();
 };
