@@ -1,0 +1,26 @@
+"""Fused acoustic substeps: runs of them leave out the halo fills in between.  Substep counts
+that are odd and even per stage, extents narrower than the halos, rows that are padded."""
+import numpy as np
+import pytest
+
+from tests import helpers
+from thunderengine_web_b200 import scenario, timestep
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('dims,nsound,align', [((5, 3, 8), 7, False), ((2, 9, 6), 8, False), ((33, 8, 5), 6, False),
+                                               ((64, 5, 13), 9, True), ((31, 40, 12), 2, False)])
+def test_fused_steps_equal_the_oracle(dims, nsound, align):
+    run = timestep.Run(scenario.tiny(*dims, dx=500.0, dz=250.0, dt=3.0, nsound=nsound, us=25.0, align_rows=align))
+    tape = run.tape(1)
+    init = run.initial_buffers()
+    cpu = helpers.cpu_run(tape, init, nsteps=2, hashes=False)
+    r = helpers.gpu_replayer(tape, init, hashes=False, mode=1)
+    r.encode_steps(2)
+    mem = r.read(r.buffers_end)
+    arena = r.base[run.rec.ids['arena']]
+    r.close()
+    for name in run.fields:
+        if name not in helpers.SCRATCH:
+            a, b = (helpers.field_view(m, run, arena, name) for m in (mem, cpu.M))
+            assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), name

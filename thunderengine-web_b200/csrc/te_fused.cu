@@ -6,9 +6,9 @@
 //
 //  * acoustic substep (timestep.js:1997-2060): acoustic_uv, acoustic_fpk,
 //    acoustic_w_solve, acoustic_pp, halo(ppd), acoustic_accumulate, halo(u, v, w)
-//    -> K1 (u/v update + u/v accumulation), K2 (pi' forcing + implicit w solve + pi'
-//       update + w accumulation, 32-column tiles staged in shared memory), K3 (the
-//       four halo fills, with the w accumulation of the halo points).
+//    -> K1 (u/v update + u/v accumulation, the w accumulation of the halo points), K2 (pi'
+//       forcing + implicit w solve + pi' update + w accumulation, 32-column tiles staged in
+//       shared memory) and, after the last substep of a run of them, K3 (the four halo fills).
 //  * runs of periodic halo fills (bc_periodic_x then bc_periodic_y per field)
 //    -> one launch for up to four fields.
 //
@@ -36,28 +36,15 @@ struct AcuArgs {
   Dims g;
   Acoustic a;
   const float *ppd, *thv, *uten, *vten, *hm;
-  float *u, *v, *w, *rru, *rrv, *rrw;
+  const float *ui, *vi;              // u, v before the substep (K1 reads these)
+  float *u, *v, *w, *rru, *rrv, *rrw;  // u, v after it
   const float *piadv, *ppten, *ppterm, *pk1, *pk2, *qk, *mm, *wten;
-  float *pp3d, *ppdw, *ppx, *cA, *cB, *sbuf;
+  float *pp3d, *ppdw, *ppx;
   float tavg;
   int saveX;
+  int wrap;  // the halos of u, v, w and ppd are the fill of the substep before, not done in memory
+  int fill;  // the last substep of a run: its halo fills are done (K3)
 };
-
-// u, v at (i, j, k) after acoustic_uv (acoustic_uv.wgsl:145-181); a point outside the
-// update range keeps its value.
-__device__ __forceinline__ float uv_u(const AcuArgs& A, int i, int j, int c) {
-  const Dims& g = A.g;
-  const float tem1 = (g.rdx * 1005.7f) * 0.5f;
-  return fmaf(A.a.dts, fmaf(-((tem1 * (A.ppd[c] - A.ppd[c - 1])) * hm_uf(g, A.hm, i)), A.thv[c] + A.thv[c - 1], A.uten[c]),
-              A.u[c]);
-}
-__device__ __forceinline__ float uv_v(const AcuArgs& A, int i, int j, int c) {
-  const Dims& g = A.g;
-  const float tem2 = (g.rdy * 1005.7f) * 0.5f;
-  const int sj = g.sJ;
-  return fmaf(A.a.dts, fmaf(-((tem2 * (A.ppd[c] - A.ppd[c - sj])) * hm_vf(g, A.hm, j)), A.thv[c] + A.thv[c - sj], A.vten[c]),
-              A.v[c]);
-}
 
 // Exact unsigned division by a divisor d >= 2 fixed for a launch: q = floor(n * m / 2^64)
 // with m = floor(2^64 / d) + 1 equals floor(n / d) for every n < 2^32 (the error term
@@ -70,87 +57,78 @@ struct FastDiv {
 static FastDiv fast_div(unsigned d) { return FastDiv{~0ull / d + 1ull, d}; }
 __device__ __forceinline__ unsigned fdiv(unsigned n, const FastDiv& f) { return (unsigned)__umul64hi(n, f.m); }
 
+// x or y index of the interior point whose value the periodic fill leaves at index i
+__device__ __forceinline__ int wrapped(int i, int n) {
+  if (i < 0) i += n;
+  else if (i >= n) i -= n;
+  return (unsigned)i < (unsigned)n ? i : ((i % n) + n) % n;  // halos wider than the domain
+}
+
 // K1: every point of the field (halos and k = nz included, as acoustic_accumulate):
 // u, v updated where acoustic_uv updates them, then rru += u, rrv += v (averaged on the
 // last substep, acoustic_accumulate.wgsl:129-158).  The points are numbered by their
-// linear index c (the field's word offset) and thread t takes c = t + q S, q < kUvLevels
-// (S a multiple of 32), so every warp reads and writes whole aligned 128-byte lines of
-// each field rather than a row segment straddling two (measured at 256x256x80: 51.5 us
-// per launch against 57.8 us for 32 x 8 blocks of two levels per thread); (i, j, k)
-// follow from c by exact division.  A thread issues all its loads before its first store
-// (the points are distinct, so nothing it stores is read by it or by another thread).
-// Row padding of aligned-row layouts (x > nx + 6) belongs to no point.
-#ifndef TE_UV_POINTS
-#define TE_UV_POINTS 1   // points per thread (2 and 4 measured slower)
-#endif
-constexpr int kUvLevels = TE_UV_POINTS;
-
-__global__ void __launch_bounds__(256) k_acu_uv_lin(AcuArgs A, FastDiv dJ, FastDiv dK, unsigned S, unsigned total) {
+// linear index c (the field's word offset), one per thread, so every warp reads and writes
+// whole aligned 128-byte lines of each field rather than a row segment straddling two
+// (measured at 256x256x80: 51.5 us per launch against 57.8 us for 32 x 8 blocks of two levels
+// per thread; two and four points per thread 55.7 / 66 us); (i, j, k) follow from c by exact
+// division.  Row padding of aligned-row layouts (x > nx + 6) belongs to no point.
+//
+// The reference fills the halos of ppd, u, v and w after every substep.  Between the substeps
+// of a run nothing but the next K1 would read those halos, and they are copies, so K1 (wrap)
+// reads each halo value at the interior point it is a copy of, and only the last substep of
+// the run does the fills (K3): per launch 9.7 us at 256x256x80, 4.4 us at 64x64x40, once per
+// stage instead of once per substep.  A halo point then reads u and v of a point that
+// another thread updates, so a wrapping K1 writes u and v to other fields than it reads
+// (ui, vi): the interior and the faces i = nx, j = ny that K2 reads.  The halo points'
+// w accumulation, which takes w before K2 of the same substep, is done here too.
+__global__ void __launch_bounds__(256) k_acu_uv_lin(AcuArgs A, FastDiv dJ, FastDiv dK, unsigned total) {
   const Dims& g = A.g;
-  const unsigned t = blockIdx.x * 256u + threadIdx.x;
-  if (t >= S) return;  // every point is some thread's t + q S
-  float un[kUvLevels], vn[kUvLevels], ru[kUvLevels], rv[kUvLevels];
-  bool on[kUvLevels], upd[kUvLevels];
-#pragma unroll
-  for (int q = 0; q < kUvLevels; q++) {
-    const unsigned c = t + q * S;
-    const unsigned kk = fdiv(c, dK);                 // level (dK: sJ * sK)
-    const unsigned r = c - kk * dK.d;
-    const unsigned jj = fdiv(r, dJ);                 // row (dJ: sJ)
-    const int x = (int)(r - jj * dJ.d);
-    const int i = x - 3, j = (int)jj - 3, k = (int)kk;
-    on[q] = c < total && x <= g.nx + 6 && j <= g.ny + 3;
-    upd[q] = on[q] && i >= 0 && j >= 0 && i <= g.nx && j <= g.ny && k < g.nz;
-    if (on[q]) {
-      un[q] = upd[q] ? uv_u(A, i, j, (int)c) : A.u[c];
-      vn[q] = upd[q] ? uv_v(A, i, j, (int)c) : A.v[c];
-      ru[q] = A.rru[c];
-      rv[q] = A.rrv[c];
-    }
+  const unsigned c = blockIdx.x * 256u + threadIdx.x;
+  if (c >= total) return;
+  const unsigned kk = fdiv(c, dK);                 // level (dK: sJ * sK)
+  const unsigned r = c - kk * dK.d;
+  const unsigned jj = fdiv(r, dJ);                 // row (dJ: sJ)
+  const int x = (int)(r - jj * dJ.d);
+  const int i = x - 3, j = (int)jj - 3, k = (int)kk;
+  if (x > g.nx + 6 || j > g.ny + 3) return;
+  const bool inner = i >= 0 && j >= 0 && i < g.nx && j < g.ny;
+  const bool upd = i >= 0 && j >= 0 && i <= g.nx && j <= g.ny && k < g.nz;
+  const int sj = g.sJ;
+  int cu = (int)c, cw = (int)c - 1, cs = (int)c - sj;  // this point, the one west and the one south of it
+  if (A.wrap && (!inner || i == 0 || j == 0)) {
+    const int iw = wrapped(i, g.nx), jw = wrapped(j, g.ny);
+    cu = gidx(g, iw, jw, k);
+    cw = gidx(g, wrapped(i - 1, g.nx), jw, k);
+    cs = gidx(g, iw, wrapped(j - 1, g.ny), k);
   }
-#pragma unroll
-  for (int q = 0; q < kUvLevels; q++) {
-    if (!on[q]) continue;
-    const unsigned c = t + q * S;
-    if (upd[q]) {
-      A.u[c] = un[q];
-      A.v[c] = vn[q];
-    }
-    if (A.tavg > 0.0f) {
-      A.rru[c] = (ru[q] + un[q]) * A.tavg;
-      A.rrv[c] = (rv[q] + vn[q]) * A.tavg;
-    } else {
-      A.rru[c] = ru[q] + un[q];
-      A.rrv[c] = rv[q] + vn[q];
-    }
+  float un = A.ui[cu], vn = A.vi[cu];
+  const float ru = A.rru[c], rv = A.rrv[c];
+  if (upd) {  // acoustic_uv.wgsl:145-181
+    const float tem1 = (g.rdx * 1005.7f) * 0.5f, tem2 = (g.rdy * 1005.7f) * 0.5f;
+    const float p = A.ppd[cu], t = A.thv[c];
+    un = fmaf(A.a.dts, fmaf(-((tem1 * (p - A.ppd[cw])) * hm_uf(g, A.hm, i)), t + A.thv[c - 1], A.uten[c]), un);
+    vn = fmaf(A.a.dts, fmaf(-((tem2 * (p - A.ppd[cs])) * hm_vf(g, A.hm, j)), t + A.thv[c - sj], A.vten[c]), vn);
   }
+  if (!inner) {
+    const float wv = A.w[cu], rr = A.rrw[c];
+    A.rrw[c] = A.tavg > 0.0f ? fmaf(wv, A.a.alph, rr) * A.tavg : rr + wv;
+  }
+  if (inner || upd) {
+    A.u[c] = un;
+    A.v[c] = vn;
+  }
+  A.rru[c] = A.tavg > 0.0f ? (ru + un) * A.tavg : ru + un;
+  A.rrv[c] = A.tavg > 0.0f ? (rv + vn) * A.tavg : rv + vn;
 }
 
 static void launch_acu_uv(const AcuArgs& A, cudaStream_t s) {
   const Dims& g = A.g;
   const unsigned total = (unsigned)g.sJ * (unsigned)g.sK * (unsigned)(g.nz + 1);
-  const unsigned S = ((total + kUvLevels - 1) / kUvLevels + 31u) / 32u * 32u;
-  launch_kernel(k_acu_uv_lin, dim3((S + 255u) / 256u), dim3(256), 0, s, A, fast_div((unsigned)g.sJ),
-                fast_div((unsigned)g.sJ * (unsigned)g.sK), S, total);
+  launch_kernel(k_acu_uv_lin, dim3((total + 255u) / 256u), dim3(256), 0, s, A, fast_div((unsigned)g.sJ),
+                fast_div((unsigned)g.sJ * (unsigned)g.sK), total);
 }
 
 // ------------------------------------------------------------ acoustic K2
-
-// Explicit pi' forcing at an interior point (acoustic_fpk.wgsl:167-207).
-__device__ __forceinline__ float fpk_at(const AcuArgs& A, int i, int j, int c, const float* w_old) {
-  const Dims& g = A.g;
-  const Acoustic& a = A.a;
-  const int sj = g.sJ, sk = g.sJ * g.sK;
-  const float temx = (a.dts * 0.5f) * g.rdx;
-  const float temy = (a.dts * 0.5f) * g.rdy;
-  const float *u = A.u, *v = A.v, *piadv = A.piadv;
-  float div = fmaf((u[c + 1] - u[c]) * g.rdx, hm_uh(g, A.hm, i), ((v[c + sj] - v[c]) * g.rdy) * hm_vh(g, A.hm, j));
-  if (fabsf(div) < a.smeps) div = 0.0f;
-  float advPi = fmaf((-fmaf(u[c], piadv[c] - piadv[c - 1], u[c + 1] * (piadv[c + 1] - piadv[c]))) * temx, hm_uh(g, A.hm, i),
-                     -((fmaf(v[c], piadv[c] - piadv[c - sj], v[c + sj] * (piadv[c + sj] - piadv[c])) * temy) * hm_vh(g, A.hm, j)));
-  return fmaf(a.beta, fmaf(w_old[c], A.pk1[c] + A.qk[c], w_old[c + sk] * (A.pk2[c] - A.qk[c])),
-              fmaf(a.dts, fmaf(-A.ppterm[c], div, A.ppten[c]), advPi));
-}
 
 // K2: a CTA owns 32 interior columns (i0..i0+31, row j) and runs their implicit w-pi'
 // solve with warp specialisation.  kLevels worker warps (one level each per pass) load
@@ -481,11 +459,6 @@ struct HaloArgs {
   Dims g;
   float* f[4];
   int nf;
-  // acoustic substep: before the fill, halo points accumulate w into rrw
-  // (acoustic_accumulate covers halos with the values they hold before the fill)
-  float* acc_w;
-  float* acc_rrw;
-  float tavg, alph;
 };
 
 // Final state of bc_periodic_x followed by bc_periodic_y (bc_periodic_x.wgsl,
@@ -513,23 +486,16 @@ __global__ void __launch_bounds__(256) k_halo_periodic(HaloArgs H) {
     const int i = col < 3 ? col - 3 : g.nx + (col - 3);
     const int ii = ((i % g.nx) + g.nx) % g.nx, jj = ((j % g.ny) + g.ny) % g.ny;
     const int dst0 = gidx(g, i, j, 0), src0 = gidx(g, ii, jj, 0);
-    const bool acc = H.acc_rrw && H.f[f] == H.acc_w;
-    float v[kHaloLevels], wv[kHaloLevels], rr[kHaloLevels];
+    float v[kHaloLevels];
 #pragma unroll
     for (int q = 0; q < kHaloLevels; q++) {
       if (k0 + q > g.nz) break;
       v[q] = H.f[f][src0 + (k0 + q) * sk];
-      if (acc) {
-        wv[q] = H.acc_w[dst0 + (k0 + q) * sk];
-        rr[q] = H.acc_rrw[dst0 + (k0 + q) * sk];
-      }
     }
 #pragma unroll
     for (int q = 0; q < kHaloLevels; q++) {
       if (k0 + q > g.nz) break;
-      const int dst = dst0 + (k0 + q) * sk;
-      if (acc) H.acc_rrw[dst] = H.tavg > 0.0f ? fmaf(wv[q], H.alph, rr[q]) * H.tavg : rr[q] + wv[q];
-      H.f[f][dst] = v[q];
+      H.f[f][dst0 + (k0 + q) * sk] = v[q];
     }
     return;
   }
@@ -540,23 +506,18 @@ __global__ void __launch_bounds__(256) k_halo_periodic(HaloArgs H) {
   const int jj = ((j % g.ny) + g.ny) % g.ny;
   const int dst0 = gidx(g, i, j, 0), src0 = gidx(g, i, jj, 0);
   // all loads of the thread's levels before the first store
-  float v[kHaloLevels][4], wv[kHaloLevels], rr[kHaloLevels];
+  float v[kHaloLevels][4];
 #pragma unroll
   for (int q = 0; q < kHaloLevels; q++) {
     if (k0 + q > g.nz) break;
 #pragma unroll
     for (int f = 0; f < 4; f++)
       if (f < H.nf) v[q][f] = H.f[f][src0 + (k0 + q) * sk];
-    if (H.acc_rrw) {
-      wv[q] = H.acc_w[dst0 + (k0 + q) * sk];
-      rr[q] = H.acc_rrw[dst0 + (k0 + q) * sk];
-    }
   }
 #pragma unroll
   for (int q = 0; q < kHaloLevels; q++) {
     if (k0 + q > g.nz) break;
     const int dst = dst0 + (k0 + q) * sk;
-    if (H.acc_rrw) H.acc_rrw[dst] = H.tavg > 0.0f ? fmaf(wv[q], H.alph, rr[q]) * H.tavg : rr[q] + wv[q];
 #pragma unroll
     for (int f = 0; f < 4; f++)
       if (f < H.nf) H.f[f][dst] = v[q][f];
@@ -1088,7 +1049,7 @@ static bool match_substep(const std::vector<Op>& ops, size_t i, FusedSegment& s,
   const float* want[3] = {u, v, w};
   for (int q = 0; q < 3; q++)
     if (!halo_pair(ops, i + 7 + 2 * q, &f) || f != want[q]) return false;
-  // the three fields K2 uses for its intermediate values must be distinct scratch
+  // the dispatches' intermediate fields, which the fused kernels do not touch, must be distinct scratch
   float *cA = ws.args.p[10], *cB = ws.args.p[11];
   if (cA == cB || cA == fpk || cB == fpk) return false;
   for (float* p : {ppd, u, v, w, pk1, pk2, qk, acc.args.p[5], acc.args.p[6], acc.args.p[7], pp.args.p[7], pp.args.p[9],
@@ -1103,9 +1064,10 @@ static bool match_substep(const std::vector<Op>& ops, size_t i, FusedSegment& s,
   A.uten = uv.args.p[4];
   A.vten = uv.args.p[5];
   A.hm = uv.args.p[30];
-  A.u = u;
-  A.v = v;
+  A.ui = A.u = u;
+  A.vi = A.v = v;
   A.w = w;
+  A.fill = 1;
   A.piadv = fp.args.p[5];
   A.ppten = fp.args.p[6];
   A.ppterm = fp.args.p[7];
@@ -1118,9 +1080,6 @@ static bool match_substep(const std::vector<Op>& ops, size_t i, FusedSegment& s,
   A.ppdw = ppd;
   A.ppx = pp.args.p[9];
   A.saveX = pp.args.iv[10];
-  A.cA = cA;
-  A.cB = cB;
-  A.sbuf = fpk;
   A.rru = acc.args.p[5];
   A.rrv = acc.args.p[6];
   A.rrw = acc.args.p[7];
@@ -1136,6 +1095,39 @@ struct FusedData {
   std::vector<HaloArgs> halo;
   std::vector<AdvArgs> adv;
 };
+
+// Runs of consecutive substeps on one set of fields skip the halo fills between them (K1).
+// u and v alternate between their fields and the two workspace fields; the first substep
+// may stay in place (it does not wrap), so that an even number of changes ends in the fields.
+static void chain_substeps(const Plan& P, std::vector<FusedSegment>& segs, std::vector<AcuArgs>& acu) {
+  auto same = [](const AcuArgs& a, const AcuArgs& b) {
+    return same_dims(a.g, b.g) && a.ppd == b.ppd && a.u == b.u && a.v == b.v && a.w == b.w && a.rru == b.rru &&
+           a.rrv == b.rrv && a.rrw == b.rrw;
+  };
+  for (size_t q = 0; q < segs.size();) {
+    size_t e = q + 1;
+    if (segs[q].kind == kAcoustic)
+      while (e < segs.size() && segs[e].kind == kAcoustic && same(acu[segs[e - 1].aux[0]], acu[segs[e].aux[0]])) e++;
+    const size_t n = e - q;
+    if (segs[q].kind == kAcoustic && n > 1 && P.work) {
+      const AcuArgs first = acu[segs[q].aux[0]];
+      float *u[2] = {first.u, P.work}, *v[2] = {first.v, P.work + P.field_stride / 4};
+      int at = 0;
+      for (size_t t = 0; t < n; t++) {
+        AcuArgs& A = acu[segs[q + t].aux[0]];
+        const int to = t == 0 && n % 2 == 1 ? 0 : at ^ 1;
+        A.ui = u[at];
+        A.vi = v[at];
+        A.u = u[to];
+        A.v = v[to];
+        A.wrap = t > 0;
+        A.fill = t + 1 == n;
+        at = to;
+      }
+    }
+    q = e;
+  }
+}
 
 void FusedStep::build(Plan& P, std::vector<Op>& ops) {
   segs.clear();
@@ -1201,6 +1193,7 @@ void FusedStep::build(Plan& P, std::vector<Op>& ops) {
     exact_to(i);
     i++;
   }
+  chain_substeps(P, segs, D.acu);
 }
 
 // The words each kernel of a fused phase reads and writes (the phase's scratch fields that
@@ -1208,7 +1201,6 @@ void FusedStep::build(Plan& P, std::vector<Op>& ops) {
 static std::vector<Access> halo_accesses(const Plan& P, const HaloArgs& H) {
   std::vector<Access> acc;
   for (int q = 0; q < H.nf; q++) acc.push_back(P.access(H.f[q], true));
-  if (H.acc_rrw) acc.push_back(P.access(H.acc_rrw, true));
   return acc;
 }
 
@@ -1239,14 +1231,14 @@ static std::vector<Access> acu_accesses(const Plan& P, const AcuArgs& A, int par
       if (f) acc.push_back(P.access(f, write));
   };
   if (part == 0) {
-    add({A.ppd, A.thv, A.uten, A.vten, A.hm}, false);
-    add({A.u, A.v, A.rru, A.rrv}, true);
+    add({A.ppd, A.thv, A.uten, A.vten, A.hm, A.ui, A.vi, A.w}, false);
+    add({A.u, A.v, A.rru, A.rrv, A.rrw}, true);
   } else if (part == 1) {
     add({A.u, A.v, A.piadv, A.ppten, A.ppterm, A.pk1, A.pk2, A.qk, A.mm, A.wten, A.hm}, false);
     add({A.w, A.pp3d, A.ppdw, A.rrw}, true);
     if (A.saveX) add({A.ppx}, true);
   } else {
-    add({A.ppdw, A.u, A.v, A.w, A.rrw}, true);
+    add({A.ppdw, A.u, A.v, A.w}, true);
   }
   return acc;
 }
@@ -1267,7 +1259,7 @@ void FusedStep::launch(Plan& P, std::vector<Op>& ops, StepDeps* deps) {
     else if (s.kind == kHalo) run(halo_accesses(P, D.halo[s.aux[0]]), q, -1);
     else if (s.kind == kAdvect) run(adv_accesses(P, D.adv[s.aux[0]], s.aux[1]), q, -1);
     else
-      for (int part = 0; part < 3; part++) run(acu_accesses(P, D.acu[s.aux[0]], part), q, part);
+      for (int part = 0; part < 2 + D.acu[s.aux[0]].fill; part++) run(acu_accesses(P, D.acu[s.aux[0]], part), q, part);
   }
 }
 
@@ -1285,7 +1277,7 @@ void FusedStep::launch_segment(Plan& P, std::vector<Op>& ops, int seg, int part)
     const Dims& g = A.g;
     if (part < 0 || part == 0) launch_acu_uv(A, P.stream);
     if (part < 0 || part == 1) launch_acu_column(A, P.stream);
-    if (part < 0 || part == 2) {
+    if (A.fill && (part < 0 || part == 2)) {
       HaloArgs H;
       std::memset(&H, 0, sizeof(H));
       H.g = g;
@@ -1294,20 +1286,15 @@ void FusedStep::launch_segment(Plan& P, std::vector<Op>& ops, int seg, int part)
       H.f[2] = A.v;
       H.f[3] = A.w;
       H.nf = 4;
-      H.acc_w = A.w;
-      H.acc_rrw = A.rrw;
-      H.tavg = A.tavg;
-      H.alph = A.a.alph;
       launch_halo(H, P.stream);
     }
   }
 }
 
-int FusedStep::launches_per_step() const {
-  if (!data) return 0;
-  int n = 0;
-  for (auto& s : segs) n += s.kind == kExact ? 0 : (s.kind == kAcoustic ? 3 : 1);
-  return n;
+int FusedStep::kernels(int seg) const {
+  const FusedSegment& s = segs.at(seg);
+  if (s.kind == kExact) return 0;
+  return s.kind == kAcoustic ? 2 + static_cast<FusedData*>(data)->acu[s.aux[0]].fill : 1;
 }
 
 void FusedStep::release() {

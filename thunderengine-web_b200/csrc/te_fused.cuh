@@ -28,7 +28,7 @@ struct FusedStep {
   void launch(Plan& P, std::vector<Op>& ops, StepDeps* deps);
   // one segment; part = -1 for all of its kernels, else the index of one of them
   void launch_segment(Plan& P, std::vector<Op>& ops, int seg, int part);
-  int launches_per_step() const;
+  int kernels(int seg) const;  // launches of a fused segment (0: a run of exact ops)
   void release();
 };
 

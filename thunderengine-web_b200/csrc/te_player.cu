@@ -456,7 +456,9 @@ int te_plan(te_ctx* ctx, const char* tape_json, size_t tape_len, const char* ker
   P.release();
   P.load_kernel_meta(kernels_json, kernels_len);
   P.plan(tape_json, tape_len, with_hashes != 0);
-  CU(cudaMalloc(&P.M, P.mem_words * 4));
+  // the word memory, then the fused steps' workspace: two fields (te_fused.cu, K1)
+  CU(cudaMalloc(&P.M, P.mem_words * 4 + 2 * P.field_stride));
+  P.work = P.field_stride ? reinterpret_cast<float*>(P.M + P.mem_words) : nullptr;
   CU(cudaMemsetAsync(P.M, 0, P.mem_words * 4, ctx->plan.stream));
   CU(cudaMalloc(&P.H, std::max<size_t>(16, (size_t)P.hash_count * 4)));
   CU(cudaMemsetAsync(P.H, 0, std::max<size_t>(16, (size_t)P.hash_count * 4), ctx->plan.stream));
@@ -680,7 +682,7 @@ int te_fused_segments(te_ctx* ctx, te_segment* out, int max, int* count) {
     out[i].kind = s.kind;
     out[i].first_op = s.first;
     out[i].last_op = s.last;
-    out[i].kernels = s.kind == 0 ? 0 : (s.kind == 1 ? 3 : 1);
+    out[i].kernels = P.fused.kernels(i);
     if (s.kind == 0)
       for (int q = s.first; q <= s.last; q++) out[i].kernels += P.active->ops[q].copy ? 0 : 1;
   }
@@ -777,7 +779,7 @@ namespace te {
 
 Access Plan::access(const void* p, bool write) const {
   const uint64_t off = (uint64_t)(static_cast<const uint32_t*>(p) - M);
-  return access_words(p, region_len(off), write);
+  return access_words(p, off < mem_words ? region_len(off) : field_stride / 4, write);  // a field of the workspace
 }
 
 std::vector<Access> Plan::accesses(const Op& o) const {
@@ -897,6 +899,7 @@ void Plan::release() {
   if (H) cudaFree(H);
   M = nullptr;
   H = nullptr;
+  work = nullptr;
   cache.clear();
   active = nullptr;
   diag_ops.clear();

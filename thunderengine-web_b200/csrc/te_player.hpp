@@ -78,6 +78,7 @@ struct Plan {
   // device
   uint32_t* M = nullptr;
   uint32_t* H = nullptr;
+  float* work = nullptr;  // two fields of workspace behind the word memory (no part of it)
   cudaGraphExec_t graph_exec = nullptr;
   cudaGraphExec_t graph_chain = nullptr;  // the chain a concurrent graph_exec replaced, which may still run
   int graph_runs = 0;             // steps launched since the step, mode or parameters last changed
