@@ -542,7 +542,7 @@ def kernel_roofline(r, run, stream, mode):
             # pk2, qk, mm, wten, pp3d, rrw; writes w, pp3d, ppd, rrw and ppx (stages 1-2: no ppx)
             stats['acoustic_column (fused fpk+w_solve+pp+accumulate)'] = [timed(lambda: r.run_segment(q, 1)), len(acu),
                                                                           18 * 4 * pts]
-            stats['halo_periodic x4 (fused)'] = [timed(lambda: r.run_segment(q, 2)), len(acu),
+            stats['halo_periodic x4 (fused)'] = [timed(lambda: r.run_segment(q, 2)), sum(segs[n][3] == 3 for n in acu),
                                                  4 * 2 * 4 * 7 * (g.strideK + g.nx) * (g.nz + 1)]
         if halo:
             q = halo[0]

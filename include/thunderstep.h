@@ -30,7 +30,7 @@ extern "C" {
 #define TE_ERANGE -5     /* offset / size outside the planned memory */
 
 /* Execution modes of te_run (te_set_mode). */
-#define TE_MODE_EXACT 0  /* one CUDA kernel per tape dispatch, reference order */
+#define TE_MODE_EXACT 0  /* every memory word as the tape's dispatches leave it */
 #define TE_MODE_FUSED 1  /* recognised step phases run as fused kernels (see te_set_mode) */
 
 /* te_config.flags */
@@ -113,10 +113,13 @@ int te_clear_hashes(te_ctx *ctx);
 /* Device address of memory word `word_off`, for callers that keep data on the GPU. */
 int te_device_ptr(te_ctx *ctx, uint64_t word_off, void **out);
 
-/* TE_MODE_EXACT (default) or TE_MODE_FUSED.  Fused mode replaces recognised phases of
+/* TE_MODE_EXACT (default) or TE_MODE_FUSED.  After a step in exact mode every memory word is
+ * the one the tape's dispatches leave, scratch included (phases whose scratch the step
+ * stores again later may run fused; te_run_ops and hash runs play one kernel per
+ * dispatch).  Fused mode replaces recognised phases of
  * the step (acoustic substeps, advection of a variable) by fused kernels; prognostic
  * fields are bit-identical to exact mode, the contents of the step's scratch fields
- * (fx, fy, fz, fpk, cA, cB, ...) are not kept.  Hash runs always use exact mode. */
+ * (fx, fy, fz, fpk, cA, cB, ...) are not kept.  Hash runs play one kernel per dispatch. */
 int te_set_mode(te_ctx *ctx, int mode);
 
 /* Fused-mode plan of the active step (built on first use): segments are runs of exact

@@ -13,12 +13,15 @@
 //    -> one launch for up to four fields.
 //
 // Contract: every field that is not step scratch (fpk, cA, cB are not written in fused
-// mode) ends bit-identical to the exact sequence.  Arithmetic per point is the
+// mode) ends bit-identical to the exact sequence; exact mode runs a phase fused only where
+// the scratch it skips is stored again later in the step (keep_final_stores).  Arithmetic per point is the
 // same sequence of binary32 operations as te_kernels.cu.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cstring>
+#include <set>
 #include <stdexcept>
 #include <string>
 
@@ -1096,6 +1099,58 @@ struct FusedData {
   std::vector<AdvArgs> adv;
 };
 
+// The words each kernel of a fused phase reads and writes (the phase's scratch fields that
+// the fused kernels do not touch left out).
+static std::vector<Access> halo_accesses(const Plan& P, const HaloArgs& H) {
+  std::vector<Access> acc;
+  for (int q = 0; q < H.nf; q++) acc.push_back(P.access(H.f[q], true));
+  return acc;
+}
+
+static std::vector<Access> adv_reads(const Plan& P, const AdvArgs& A, int kind) {
+  std::vector<Access> acc;
+  const FluxNames* fs = nullptr;
+  for (auto& c : kFluxSets)
+    if (c.kind == kind) fs = &c;
+  for (int b = 0; b < kMaxBind; b++) {
+    if (b != fs->out_h && A.fx.p[b]) acc.push_back(P.access(A.fx.p[b], false));
+    if (b != fs->out_h && A.fy.p[b]) acc.push_back(P.access(A.fy.p[b], false));
+    if (b != fs->out_z && A.fz.p[b]) acc.push_back(P.access(A.fz.p[b], false));
+    if (b != 3 && b != 4 && b != 5 && b != 11 && b != 19 && A.as.p[b]) acc.push_back(P.access(A.as.p[b], false));
+  }
+  for (const float* f : {A.div3d, A.thterm, A.phiA})
+    if (f) acc.push_back(P.access(f, false));
+  return acc;
+}
+
+static std::vector<Access> adv_accesses(const Plan& P, const AdvArgs& A, int kind) {
+  std::vector<Access> acc = adv_reads(P, A, kind);
+  // an RK update that keeps its tendency to itself still reads it on open u, v edges
+  acc.push_back(P.access(A.dest, A.accumulate || A.write_dest));
+  for (float* f : {A.phi, A.fxo, A.fyo, A.fzo})
+    if (f) acc.push_back(P.access(f, true));
+  return acc;
+}
+
+static std::vector<Access> acu_accesses(const Plan& P, const AcuArgs& A, int part) {
+  std::vector<Access> acc;
+  auto add = [&](std::initializer_list<const float*> fields, bool write) {
+    for (const float* f : fields)
+      if (f) acc.push_back(P.access(f, write));
+  };
+  if (part == 0) {
+    add({A.ppd, A.thv, A.uten, A.vten, A.hm, A.ui, A.vi, A.w}, false);
+    add({A.u, A.v, A.rru, A.rrv, A.rrw}, true);
+  } else if (part == 1) {
+    add({A.u, A.v, A.piadv, A.ppten, A.ppterm, A.pk1, A.pk2, A.qk, A.mm, A.wten, A.hm}, false);
+    add({A.w, A.pp3d, A.ppdw, A.rrw}, true);
+    if (A.saveX) add({A.ppx}, true);
+  } else {
+    add({A.ppdw, A.u, A.v, A.w}, true);
+  }
+  return acc;
+}
+
 // Runs of consecutive substeps on one set of fields skip the halo fills between them (K1).
 // u and v alternate between their fields and the two workspace fields; the first substep
 // may stay in place (it does not wrap), so that an even number of changes ends in the fields.
@@ -1129,7 +1184,121 @@ static void chain_substeps(const Plan& P, std::vector<FusedSegment>& segs, std::
   }
 }
 
-void FusedStep::build(Plan& P, std::vector<Op>& ops) {
+// What a fused phase leaves out: the output `out` of op `op`.
+struct Skipped {
+  int op;
+  const float* out;
+};
+
+static std::vector<Skipped> skipped_stores(const std::vector<Op>& ops, const FusedSegment& s, const FusedData& D) {
+  std::vector<Skipped> v;
+  if (s.kind == kAcoustic) {
+    const Op &fp = ops[s.first + 1], &ws = ops[s.first + 2];
+    v = {{s.first + 1, fp.args.p[11]}, {s.first + 2, ws.args.p[10]}, {s.first + 2, ws.args.p[11]}};
+  } else if (s.kind == kAdvect) {
+    const AdvArgs& A = D.adv[s.aux[0]];
+    if (!A.fxo)
+      for (int q = 0; q < 3; q++) v.push_back({s.first + q, ops[s.first + 3].args.p[3 + q]});
+    if (!A.accumulate && !A.write_dest) v.push_back({s.first + 3, A.dest});
+  }
+  return v;
+}
+
+// Two dispatches with equal keys write the same words: same kernel, output field, dispatch
+// grid, dimensions and (adv_assemble) stagger.
+typedef std::array<long long, 11> StoreKey;
+static StoreKey store_key(const Op& o, const float* out) {
+  const Dims& g = o.args.g;
+  return StoreKey{(long long)(uintptr_t)o.spec, (long long)(uintptr_t)out, o.grid[0], o.grid[1], o.grid[2], g.nx, g.ny, g.nz,
+                  g.sJ, g.sK, o.name == "adv_assemble" ? o.args.iv[1] : 0};
+}
+
+// The regions the ops of a phase bind are equal or disjoint, and nothing a phase's fused
+// kernels write or skip is read by them in another role.
+static bool plain_bindings(const Plan& P, const std::vector<Op>& ops, const std::vector<std::vector<Access>>& acc,
+                           const FusedSegment& s, const FusedData& D) {
+  std::vector<Access> all;
+  for (int q = s.first; q <= s.last; q++) all.insert(all.end(), acc[q].begin(), acc[q].end());
+  std::sort(all.begin(), all.end(), [](const Access& a, const Access& b) { return a.lo < b.lo; });
+  for (size_t q = 1; q < all.size(); q++)
+    if (all[q].lo != all[q - 1].lo && all[q].lo < all[q - 1].hi) return false;
+  std::vector<const float*> wr, rd;
+  if (s.kind == kAcoustic) {
+    const AcuArgs& A = D.acu[s.aux[0]];
+    const Op &fp = ops[s.first + 1], &ws = ops[s.first + 2];
+    wr = {A.ppd, A.u, A.v, A.w, A.rru, A.rrv, A.rrw, A.pp3d, A.ppx, fp.args.p[11], ws.args.p[10], ws.args.p[11]};
+    rd = {A.thv, A.uten, A.vten, A.hm, A.piadv, A.ppten, A.ppterm, A.pk1, A.pk2, A.qk, A.mm, A.wten};
+    if (A.ppd != A.ppdw) return false;
+  } else if (s.kind == kAdvect) {
+    const AdvArgs& A = D.adv[s.aux[0]];
+    const KArgs& as = ops[s.first + 3].args;
+    wr = {A.dest, as.p[3], as.p[4], as.p[5]};
+    if (A.phi) wr.push_back(A.phi);
+    for (const Access& a : adv_reads(P, A, s.aux[1])) rd.push_back(reinterpret_cast<const float*>(a.lo));
+  }
+  std::sort(wr.begin(), wr.end());
+  for (size_t q = 0; q < wr.size(); q++) {
+    if (!wr[q] || (q && wr[q] == wr[q - 1])) return false;
+    for (const float* r : rd)
+      if (r == wr[q]) return false;
+  }
+  return true;
+}
+
+// keep_scratch (exact mode): a phase stays fused when every store it skips is made again later in the step,
+// by a dispatch that writes the same words, before anything else touches the field.  The
+// last dispatch of each kind is then one that runs (or a fused phase that stores its
+// fluxes), so every word ends with the value of its last writer.  Of a moist step the last
+// substep and the last variable of each flux kind run per dispatch (333 launches -> 157).
+// One B200, per step: exact 128x128x64 1.58 -> 1.26 ms, exact 12x10x8 280 -> 197 us; the
+// per-dispatch form spent the difference on launches and on writing and re-reading fluxes.
+static void keep_final_stores(const Plan& P, const std::vector<Op>& ops, std::vector<FusedSegment>& segs, const FusedData& D) {
+  std::vector<std::vector<Access>> acc;
+  for (const Op& o : ops) acc.push_back(P.accesses(o));
+  std::set<StoreKey> later;  // keys of the stores that segments after this one make
+  auto add = [&](const Op& o) {
+    if (o.copy || !o.spec) return;
+    for (int q = 0; q < o.spec->nparams; q++) {
+      const ParamSpec& ps = o.spec->params[q];
+      if (ps.kind == kPtr && ps.write && o.args.p[ps.index]) later.insert(store_key(o, o.args.p[ps.index]));
+    }
+  };
+  for (size_t n = segs.size(); n-- > 0;) {
+    FusedSegment& s = segs[n];
+    bool keep = s.kind == kExact || plain_bindings(P, ops, acc, s, D);
+    if (keep && s.kind != kExact) {
+      for (const Skipped& k : skipped_stores(ops, s, D)) {
+        const StoreKey key = store_key(ops[k.op], k.out);
+        if (!later.count(key)) keep = false;
+        const Access f = P.access(k.out, true);
+        for (size_t q = (size_t)s.last + 1; keep && q < ops.size(); q++) {
+          bool touched = false;
+          for (const Access& a : acc[q]) touched |= a.lo < f.hi && f.lo < a.hi;
+          if (!touched) continue;
+          // the first op that touches the field writes it without reading it
+          keep = !ops[q].copy && (store_key(ops[q], k.out) == key || writes_first(ops[q], k.out));
+          break;
+        }
+        if (!keep) break;
+      }
+    }
+    if (!keep) s.kind = kExact;
+    if (s.kind == kExact) {
+      for (int q = s.first; q <= s.last; q++) add(ops[q]);
+    } else if (s.kind == kAdvect && D.adv[s.aux[0]].fxo) {
+      for (int q = 0; q < 3; q++) add(ops[s.first + q]);
+    }
+  }
+  // adjacent exact runs in one
+  std::vector<FusedSegment> out;
+  for (const FusedSegment& s : segs) {
+    if (s.kind == kExact && !out.empty() && out.back().kind == kExact) out.back().last = s.last;
+    else out.push_back(s);
+  }
+  segs.swap(out);
+}
+
+void FusedStep::build(Plan& P, std::vector<Op>& ops, bool keep_scratch) {
   segs.clear();
   if (!data) data = new FusedData();
   FusedData& D = *static_cast<FusedData*>(data);
@@ -1193,54 +1362,8 @@ void FusedStep::build(Plan& P, std::vector<Op>& ops) {
     exact_to(i);
     i++;
   }
+  if (keep_scratch) keep_final_stores(P, ops, segs, D);
   chain_substeps(P, segs, D.acu);
-}
-
-// The words each kernel of a fused phase reads and writes (the phase's scratch fields that
-// the fused kernels do not touch left out).
-static std::vector<Access> halo_accesses(const Plan& P, const HaloArgs& H) {
-  std::vector<Access> acc;
-  for (int q = 0; q < H.nf; q++) acc.push_back(P.access(H.f[q], true));
-  return acc;
-}
-
-static std::vector<Access> adv_accesses(const Plan& P, const AdvArgs& A, int kind) {
-  std::vector<Access> acc;
-  const FluxNames* fs = nullptr;
-  for (auto& c : kFluxSets)
-    if (c.kind == kind) fs = &c;
-  for (int b = 0; b < kMaxBind; b++) {
-    if (b != fs->out_h && A.fx.p[b]) acc.push_back(P.access(A.fx.p[b], false));
-    if (b != fs->out_h && A.fy.p[b]) acc.push_back(P.access(A.fy.p[b], false));
-    if (b != fs->out_z && A.fz.p[b]) acc.push_back(P.access(A.fz.p[b], false));
-    if (b != 3 && b != 4 && b != 5 && b != 11 && b != 19 && A.as.p[b]) acc.push_back(P.access(A.as.p[b], false));
-  }
-  for (const float* f : {A.div3d, A.thterm, A.phiA})
-    if (f) acc.push_back(P.access(f, false));
-  // an RK update that keeps its tendency to itself still reads it on open u, v edges
-  acc.push_back(P.access(A.dest, A.accumulate || A.write_dest));
-  for (float* f : {A.phi, A.fxo, A.fyo, A.fzo})
-    if (f) acc.push_back(P.access(f, true));
-  return acc;
-}
-
-static std::vector<Access> acu_accesses(const Plan& P, const AcuArgs& A, int part) {
-  std::vector<Access> acc;
-  auto add = [&](std::initializer_list<const float*> fields, bool write) {
-    for (const float* f : fields)
-      if (f) acc.push_back(P.access(f, write));
-  };
-  if (part == 0) {
-    add({A.ppd, A.thv, A.uten, A.vten, A.hm, A.ui, A.vi, A.w}, false);
-    add({A.u, A.v, A.rru, A.rrv, A.rrw}, true);
-  } else if (part == 1) {
-    add({A.u, A.v, A.piadv, A.ppten, A.ppterm, A.pk1, A.pk2, A.qk, A.mm, A.wten, A.hm}, false);
-    add({A.w, A.pp3d, A.ppdw, A.rrw}, true);
-    if (A.saveX) add({A.ppx}, true);
-  } else {
-    add({A.ppdw, A.u, A.v, A.w}, true);
-  }
-  return acc;
 }
 
 void FusedStep::launch(Plan& P, std::vector<Op>& ops, StepDeps* deps) {

@@ -23,7 +23,9 @@ struct FusedSegment {
 struct FusedStep {
   std::vector<FusedSegment> segs;
   void* data = nullptr;  // kernel arguments of the fused segments
-  void build(Plan& P, std::vector<Op>& ops);
+  // with keep_scratch every word of memory ends as the op sequence leaves it: a phase whose
+  // fused kernels skip scratch stores runs per dispatch unless the step stores them again later
+  void build(Plan& P, std::vector<Op>& ops, bool keep_scratch);
   // the whole step; with deps (during a capture) each kernel after those it depends on only
   void launch(Plan& P, std::vector<Op>& ops, StepDeps* deps);
   // one segment; part = -1 for all of its kernels, else the index of one of them

@@ -468,7 +468,7 @@ int te_plan(te_ctx* ctx, const char* tape_json, size_t tape_len, const char* ker
   P.bytes_init.clear();
   P.finalize_args(P.active->ops);
   P.finalize_args(P.diag_ops);
-  P.fused_dirty = true;
+  P.fused_dirty = P.exact_dirty = true;
   API_END(ctx)
 }
 
@@ -672,7 +672,7 @@ int te_fused_segments(te_ctx* ctx, te_segment* out, int max, int* count) {
   require_plan(ctx);
   te::Plan& P = ctx->plan;
   if (P.fused_dirty || P.fused.segs.empty()) {
-    P.fused.build(P, P.active->ops);
+    P.fused.build(P, P.active->ops, false);
     P.fused_dirty = false;
   }
   int n = (int)P.fused.segs.size();
@@ -695,7 +695,7 @@ int te_run_segment(te_ctx* ctx, int seg, int part) {
   CU(cudaSetDevice(ctx->device));
   te::Plan& P = ctx->plan;
   if (P.fused_dirty || P.fused.segs.empty()) {
-    P.fused.build(P, P.active->ops);
+    P.fused.build(P, P.active->ops, false);
     P.fused_dirty = false;
   }
   if (seg < 0 || seg >= (int)P.fused.segs.size()) throw te::ApiError(TE_EINVAL, "segment out of range");
@@ -837,21 +837,24 @@ void Plan::invalidate_graphs() {
   graph_exec = graph_chain = nullptr;
   graph_runs = 0;
   graph_concurrent = false;
-  fused_dirty = true;
+  fused_dirty = exact_dirty = true;
 }
 
 cudaGraph_t Plan::capture_step(bool concurrent) {
   if (mode == TE_MODE_FUSED && fused_dirty) {
-    fused.build(*this, active->ops);
+    fused.build(*this, active->ops, false);
     fused_dirty = false;
+  }
+  if (mode == TE_MODE_EXACT && exact_dirty) {
+    exact_fused.build(*this, active->ops, true);
+    exact_dirty = false;
   }
   cudaGraph_t graph = nullptr;
   CU(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
   try {
     StepDeps deps(stream);
     StepDeps* dp = concurrent ? &deps : nullptr;
-    if (mode == TE_MODE_FUSED) fused.launch(*this, active->ops, dp);
-    else launch_exact(active->ops, 0, (int)active->ops.size() - 1, false, dp);
+    (mode == TE_MODE_FUSED ? fused : exact_fused).launch(*this, active->ops, dp);
     if (dp) CU(deps.finish());
   } catch (...) {
     cudaStreamEndCapture(stream, &graph);
@@ -895,6 +898,7 @@ void Plan::release() {
   release_adjoint(*this);
   invalidate_graphs();
   fused.release();
+  exact_fused.release();
   if (M) cudaFree(M);
   if (H) cudaFree(H);
   M = nullptr;

@@ -83,8 +83,9 @@ struct Plan {
   cudaGraphExec_t graph_chain = nullptr;  // the chain a concurrent graph_exec replaced, which may still run
   int graph_runs = 0;             // steps launched since the step, mode or parameters last changed
   bool graph_concurrent = false;  // graph_exec holds the data's orders only, not the whole chain
-  FusedStep fused;
-  bool fused_dirty = true;
+  FusedStep fused;        // the active step in fused mode
+  FusedStep exact_fused;  // in exact mode: the phases whose every store the step repeats, fused
+  bool fused_dirty = true, exact_dirty = true;
   AdjointState* adjoint = nullptr;  // checkpoints, undo log and adjoint memory of te_adjoint_*
 
   void load_kernel_meta(const char* kjson, size_t klen);
