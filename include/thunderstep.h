@@ -220,8 +220,8 @@ typedef struct te_wsolve_fields {
  * allocate device memory where they run the solve (their pool belongs to another
  * allocator, or the host process forbids allocation after start-up).  It computes the
  * same w as the tape kernel acoustic_w_solve (bit for bit) but keeps the Thomas
- * coefficients, which the tape writes to the arena fields cA and cB, in a fixed 64 MiB
- * array inside this library; it allocates nothing.
+ * coefficients, which the tape writes to the arena fields cA and cB, in shared memory up to
+ * nz = 200 and in a fixed 64 MiB array inside this library above; it allocates nothing.
  *   - Limit: nx * ny * (nz - 2) <= 8,388,608 (256 x 256 columns up to nz = 130) and
  *     ny <= 262,140; larger grids, nz < 3 or a NULL field return TE_ERANGE / TE_EINVAL
  *     with a message in `err` (`err_len` bytes, may be NULL) and launch nothing.
