@@ -9,8 +9,8 @@
 // logged) and running the op's adjoint operator (te_adjoint.cuh), which turns the
 // adjoints of the values after the op into the adjoints of the values before it.  At the
 // end memory holds the state of step 0 and the adjoint memory the gradient with respect
-// to it.  Each block position has its own CUDA graph for the logged replay and for the
-// reverse walk, so a step costs two graph launches.
+// to it.  One CUDA graph is the logged replay of a step and one its reverse walk, so a step costs
+// two graph launches.
 //
 // The adjoint memory has the layout of the player's word memory: the adjoint of the value
 // at word w is the float at word w.
@@ -199,48 +199,88 @@ struct AdjEntry {
   const char* name;
   AdjLaunch launch;
   uint64_t reads;
+  // bindings whose adjoints the operator reads and writes, and those it only adds to with
+  // atomics (operators that add to the same adjoints need no order between them)
+  uint64_t owns, adds;
 };
 
 #define B1(n) (uint64_t(1) << (n))
 static const AdjEntry kAdjTable[] = {
-    {"adv_flux_x", launch_adj<OpFluxX>, B1(1) | B1(2)},
-    {"adv_flux_y", launch_adj<OpFluxY>, B1(1) | B1(2)},
-    {"adv_flux_z", launch_adj<OpFluxZ>, B1(1) | B1(2) | B1(3) | B1(4)},
-    {"adv_flux_x_stag", launch_adj<OpStagX>, B1(2) | B1(3) | B1(4) | B1(7)},
-    {"adv_flux_y_stag", launch_adj<OpStagY>, B1(2) | B1(3) | B1(4) | B1(7)},
-    {"adv_flux_z_stag", launch_adj<OpStagZ>, B1(2) | B1(5) | B1(6) | B1(7)},
-    {"adv_flux_x_weno", launch_adj<OpWenoX>, B1(1) | B1(2)},
-    {"adv_flux_y_weno", launch_adj<OpWenoY>, B1(1) | B1(2)},
-    {"adv_flux_z_weno", launch_adj<OpWenoZ>, B1(1) | B1(2) | B1(3) | B1(4)},
-    {"adv_flux_x_weno_uv", launch_adj<OpWenoUvX>, B1(2) | B1(3)},
-    {"adv_flux_y_weno_uv", launch_adj<OpWenoUvY>, B1(2) | B1(3)},
-    {"adv_flux_z_weno_uv", launch_adj<OpWenoUvZ>, B1(2) | B1(3) | B1(4) | B1(5)},
-    {"adv_flux_x_weno_w", launch_adj<OpWenoWX>, B1(1) | B1(2) | B1(3)},
-    {"adv_flux_y_weno_w", launch_adj<OpWenoWY>, B1(1) | B1(2) | B1(3)},
-    {"adv_flux_z_weno_w", launch_adj<OpWenoWZ>, B1(1) | B1(2)},
-    {"adv_assemble", launch_adj<OpAssemble>, B1(2) | B1(6) | B1(7) | B1(8) | B1(9) | B1(10) | B1(15) | B1(16) | B1(30)},
-    {"rk_update", launch_adj<OpRk>, 0},
-    {"apply_thterm", launch_adj<OpThterm>, B1(1) | B1(2)},
-    {"buoyancy_apply", launch_adj<OpBuoy>, B1(2) | B1(3)},
+    {"adv_flux_x", launch_adj<OpFluxX>, B1(1) | B1(2),
+     B1(3), B1(1) | B1(2)},
+    {"adv_flux_y", launch_adj<OpFluxY>, B1(1) | B1(2),
+     B1(3), B1(1) | B1(2)},
+    {"adv_flux_z", launch_adj<OpFluxZ>, B1(1) | B1(2) | B1(3) | B1(4),
+     B1(5), B1(1) | B1(2)},
+    {"adv_flux_x_stag", launch_adj<OpStagX>, B1(2) | B1(3) | B1(4) | B1(7),
+     B1(8), B1(2) | B1(3)},
+    {"adv_flux_y_stag", launch_adj<OpStagY>, B1(2) | B1(3) | B1(4) | B1(7),
+     B1(8), B1(2) | B1(4)},
+    {"adv_flux_z_stag", launch_adj<OpStagZ>, B1(2) | B1(5) | B1(6) | B1(7),
+     B1(8), B1(2) | B1(5)},
+    {"adv_flux_x_weno", launch_adj<OpWenoX>, B1(1) | B1(2),
+     B1(5), B1(1) | B1(2)},
+    {"adv_flux_y_weno", launch_adj<OpWenoY>, B1(1) | B1(2),
+     B1(5), B1(1) | B1(2)},
+    {"adv_flux_z_weno", launch_adj<OpWenoZ>, B1(1) | B1(2) | B1(3) | B1(4),
+     B1(8), B1(1) | B1(2)},
+    {"adv_flux_x_weno_uv", launch_adj<OpWenoUvX>, B1(2) | B1(3),
+     B1(5), B1(2) | B1(3)},
+    {"adv_flux_y_weno_uv", launch_adj<OpWenoUvY>, B1(2) | B1(3),
+     B1(5), B1(2) | B1(3)},
+    {"adv_flux_z_weno_uv", launch_adj<OpWenoUvZ>, B1(2) | B1(3) | B1(4) | B1(5),
+     B1(7), B1(2) | B1(3)},
+    {"adv_flux_x_weno_w", launch_adj<OpWenoWX>, B1(1) | B1(2) | B1(3),
+     B1(5), B1(1) | B1(2)},
+    {"adv_flux_y_weno_w", launch_adj<OpWenoWY>, B1(1) | B1(2) | B1(3),
+     B1(5), B1(1) | B1(2)},
+    {"adv_flux_z_weno_w", launch_adj<OpWenoWZ>, B1(1) | B1(2),
+     B1(4), B1(1) | B1(2)},
+    {"adv_assemble", launch_adj<OpAssemble>, B1(2) | B1(6) | B1(7) | B1(8) | B1(9) | B1(10) | B1(15) | B1(16) | B1(30),
+     B1(11), B1(2) | B1(3) | B1(4) | B1(5) | B1(6)},
+    {"rk_update", launch_adj<OpRk>, 0,
+     B1(2) | B1(3) | B1(4), 0},
+    {"apply_thterm", launch_adj<OpThterm>, B1(1) | B1(2),
+     B1(1) | B1(3), 0},
+    {"buoyancy_apply", launch_adj<OpBuoy>, B1(2) | B1(3),
+     B1(4), B1(1)},
     {"update_diagnostics_moist", launch_adj<OpDiag>,
-     B1(3) | B1(4) | B1(8) | B1(9) | B1(10) | B1(11) | B1(12) | B1(13) | B1(14)},
-    {"stage_tendency_reset", launch_adj<OpTendReset>, 0},
-    {"massflux_from_state", launch_adj<OpMassflux>, B1(4) | B1(5)},
-    {"div_massflux", launch_adj<OpDivMassflux>, B1(4) | B1(30)},
-    {"divergence3d", launch_adj<OpDiv3d>, B1(1) | B1(2) | B1(3) | B1(4) | B1(30)},
-    {"velocity_to_massflux", launch_adj<OpVelMassflux>, B1(1) | B1(2)},
-    {"build_sadv", launch_adj<OpSadv>, 0},
-    {"stage_state_reset", launch_adj<OpStateReset>, 0},
-    {"acoustic_begin", launch_adj<OpBegin>, 0},
-    {"acoustic_prepare", launch_adj<OpPrepare>, 0},
-    {"acoustic_uv", launch_adj<OpUv>, B1(2) | B1(3) | B1(30)},
-    {"acoustic_fpk", launch_adj<OpFpk>, B1(2) | B1(3) | B1(5) | B1(7) | B1(8) | B1(9) | B1(10) | B1(30)},
-    {"acoustic_pp", launch_adj<OpPp>, B1(2) | B1(3) | B1(4) | B1(5) | B1(6) | B1(7)},
-    {"acoustic_accumulate", launch_adj<OpAccum>, 0},
-    {"bc_periodic_x", launch_adj_halo<OpHaloX>, 0},
-    {"bc_periodic_y", launch_adj_halo<OpHaloY>, 0},
-    {"ppx_finish", launch_adj<OpPpxFinish>, 0},
-    {"acoustic_w_solve", launch_adj_wsolve, B1(2) | B1(3) | B1(4) | B1(5)},
+     B1(3) | B1(4) | B1(8) | B1(9) | B1(10) | B1(11) | B1(12) | B1(13) | B1(14),
+     B1(1) | B1(2) | B1(15) | B1(16) | B1(17) | B1(18) | B1(19), 0},
+    {"stage_tendency_reset", launch_adj<OpTendReset>, 0,
+     B1(1) | B1(2) | B1(3), 0},
+    {"massflux_from_state", launch_adj<OpMassflux>, B1(4) | B1(5),
+     B1(1) | B1(2) | B1(3) | B1(6) | B1(7) | B1(8), 0},
+    {"div_massflux", launch_adj<OpDivMassflux>, B1(4) | B1(30),
+     B1(5), B1(1) | B1(2) | B1(3)},
+    {"divergence3d", launch_adj<OpDiv3d>, B1(1) | B1(2) | B1(3) | B1(4) | B1(30),
+     B1(5), B1(1) | B1(2) | B1(3)},
+    {"velocity_to_massflux", launch_adj<OpVelMassflux>, B1(1) | B1(2),
+     B1(3) | B1(4) | B1(5), 0},
+    {"build_sadv", launch_adj<OpSadv>, 0,
+     B1(2) | B1(3), 0},
+    {"stage_state_reset", launch_adj<OpStateReset>, 0,
+     B1(1) | B1(2) | B1(3) | B1(4) | B1(5) | B1(6) | B1(7) | B1(8) | B1(9) | B1(10), 0},
+    {"acoustic_begin", launch_adj<OpBegin>, 0,
+     B1(2) | B1(3) | B1(4) | B1(5), 0},
+    {"acoustic_prepare", launch_adj<OpPrepare>, 0,
+     B1(11) | B1(12) | B1(13) | B1(14), 0},
+    {"acoustic_uv", launch_adj<OpUv>, B1(2) | B1(3) | B1(30),
+     B1(4) | B1(5) | B1(6) | B1(7), B1(2)},
+    {"acoustic_fpk", launch_adj<OpFpk>, B1(2) | B1(3) | B1(5) | B1(7) | B1(8) | B1(9) | B1(10) | B1(30),
+     B1(6) | B1(11), B1(2) | B1(3) | B1(4)},
+    {"acoustic_pp", launch_adj<OpPp>, B1(2) | B1(3) | B1(4) | B1(5) | B1(6) | B1(7),
+     B1(7) | B1(8) | B1(9), B1(2) | B1(6)},
+    {"acoustic_accumulate", launch_adj<OpAccum>, 0,
+     B1(2) | B1(3) | B1(4) | B1(5) | B1(6) | B1(7), 0},
+    {"bc_periodic_x", launch_adj_halo<OpHaloX>, 0,
+     B1(1), 0},
+    {"bc_periodic_y", launch_adj_halo<OpHaloY>, 0,
+     B1(1), 0},
+    {"ppx_finish", launch_adj<OpPpxFinish>, 0,
+     B1(1) | B1(2), 0},
+    {"acoustic_w_solve", launch_adj_wsolve, B1(2) | B1(3) | B1(4) | B1(5),
+     B1(6) | B1(7) | B1(8) | B1(9) | B1(10) | B1(11), 0},
 };
 #undef B1
 
@@ -318,22 +358,33 @@ static void launch_adj_halo_run(const HaloRunArgs& H, cudaStream_t s) {
 
 // The undo log's copies of one op's regions in one launch: region q is `rows` rows of
 // `width` words, `pitch` words apart, at word `off` of the memory, packed at word `log` of
-// the undo log; `start` holds the prefix sums of the regions' sizes.  save: memory -> log,
-// restore: log -> memory.
+// the step's part of the undo log, which starts at word *at (one graph serves every step of a
+// block: the host moves *at between launches).  A contiguous region that is aligned moves
+// 16 bytes per thread (whole fields), the
+// halo strips one word.  `start` holds the prefix sums of the regions' sizes in those units.
+// save: memory -> log, restore: log -> memory.
 constexpr int kCopyBatch = 8;
 struct CopyBatch {
   uint64_t off[kCopyBatch], pitch[kCopyBatch], log[kCopyBatch];
   uint32_t width[kCopyBatch], rows[kCopyBatch];
   uint32_t start[kCopyBatch + 1];
+  uint32_t vec[kCopyBatch];
   int n;
 };
 
-__global__ void __launch_bounds__(256) k_batch_copy(uint32_t* M, uint32_t* L, CopyBatch B, int restore) {
+__global__ void __launch_bounds__(256) k_batch_copy(uint32_t* M, uint32_t* undo, const uint64_t* at, CopyBatch B, int restore) {
   const uint32_t total = B.start[B.n];
+  uint32_t* L = undo + *at;
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
     int q = 0;
     while (q + 1 < B.n && t >= B.start[q + 1]) q++;
     const uint32_t e = t - B.start[q];
+    if (B.vec[q]) {
+      uint4 *m = reinterpret_cast<uint4*>(M + B.off[q]) + e, *l = reinterpret_cast<uint4*>(L + B.log[q]) + e;
+      if (restore) *m = *l;
+      else *l = *m;
+      continue;
+    }
     uint64_t m;
     if (B.rows[q] == 1) {
       m = B.off[q] + e;
@@ -347,6 +398,8 @@ __global__ void __launch_bounds__(256) k_batch_copy(uint32_t* M, uint32_t* L, Co
   }
 }
 
+__global__ void k_set_word(uint64_t* p, uint64_t v) { *p = v; }
+
 }  // namespace adj
 
 // A written region in words: `rows` rows of `width` words, `pitch` words apart.
@@ -354,6 +407,7 @@ struct Region {
   uint64_t off, width, pitch, rows;
   uint64_t field;  // word offset of the field (binding) the region belongs to
   uint64_t size() const { return width * rows; }
+  uint64_t logged() const { return (size() + 3) / 4 * 4; }  // its words of the undo log: regions start 16-byte aligned
   uint64_t last() const { return off + (rows - 1) * pitch + width - 1; }
   // every word of r lies in this region (a contiguous region, or the same pitched strip)
   bool covers(const Region& r) const {
@@ -374,7 +428,15 @@ struct AdjointState {
   uint64_t step_undo_words = 0;
   uint32_t* undo = nullptr;
   uint64_t undo_cap = 0;  // words
-  std::vector<cudaGraphExec_t> fwd_graph, rev_graph;  // per position in a block
+  uint64_t* log_at = nullptr;  // device: where the current step's part of the undo log starts
+  // logged replay and reverse walk of a step: a chain of its launches for the first
+  // kChainLaunches, then with the orders the data needs (te_deps.hpp)
+  struct StepGraph {
+    cudaGraphExec_t exec = nullptr, chain = nullptr;
+    int launches = 0;
+    bool concurrent = false;
+  };
+  StepGraph fwd_graph, rev_graph;
   // runs of periodic halo pairs (ops first..last) replayed and reversed as one launch each
   struct HaloRun {
     int first = 0, last = 0, nf = 0;
@@ -386,12 +448,11 @@ struct AdjointState {
   std::vector<int> run_from, run_to;  // per op: the run it starts / ends, or -1
 
   void drop_graphs() {
-    for (auto g : fwd_graph)
-      if (g) cudaGraphExecDestroy(g);
-    for (auto g : rev_graph)
-      if (g) cudaGraphExecDestroy(g);
-    fwd_graph.clear();
-    rev_graph.clear();
+    for (StepGraph* g : {&fwd_graph, &rev_graph}) {
+      if (g->exec) cudaGraphExecDestroy(g->exec);
+      if (g->chain) cudaGraphExecDestroy(g->chain);
+      *g = StepGraph();
+    }
   }
 };
 
@@ -402,6 +463,7 @@ void release_adjoint(Plan& P) {
   for (auto p : S->ckpt) cudaFree(p);
   if (S->L) cudaFree(S->L);
   if (S->undo) cudaFree(S->undo);
+  if (S->log_at) cudaFree(S->log_at);
   delete S;
   P.adjoint = nullptr;
 }
@@ -425,6 +487,14 @@ AdjointState& state(Plan& P) {
 }
 
 uint64_t regions_words(const std::vector<Region>& regs);
+
+// Launches: in a concurrent capture after what they depend on, else in stream order.
+template <class F>
+void in_order(StepDeps* deps, const std::vector<Access>& acc, F launch) {
+  if (deps) ACU(deps->run(acc, launch));
+  else launch();
+  ACU(cudaGetLastError());
+}
 
 // Per-op tables of the active step: written regions, adjoint arguments and operators.
 void build_tables(Plan& P, AdjointState& S) {
@@ -562,12 +632,13 @@ void build_tables(Plan& P, AdjointState& S) {
   S.step = P.active;
 }
 
-// Saves the regions of op `i` of the memory in the undo log from word `cur` on, or restores
+// Saves the regions of one op in the undo log from word `cur` of the step's part on, or restores
 // them from there (k_batch_copy: one launch for up to kCopyBatch regions).
-void copy_regions(Plan& P, const std::vector<Region>& regs, uint32_t* log, uint64_t cur, bool restore) {
+void copy_regions(Plan& P, AdjointState& S, const std::vector<Region>& regs, uint64_t cur, bool restore, StepDeps* deps) {
   for (size_t q0 = 0; q0 < regs.size(); q0 += adj::kCopyBatch) {
     adj::CopyBatch B;
     std::memset(&B, 0, sizeof B);
+    std::vector<Access> acc;
     uint64_t total = 0;
     for (size_t q = q0; q < regs.size() && B.n < adj::kCopyBatch; q++) {
       const Region& r = regs[q];
@@ -577,28 +648,32 @@ void copy_regions(Plan& P, const std::vector<Region>& regs, uint32_t* log, uint6
       B.width[B.n] = (uint32_t)r.width;
       B.rows[B.n] = (uint32_t)r.rows;
       B.start[B.n] = (uint32_t)total;
+      B.vec[B.n] = r.rows == 1 && r.off % 4 == 0 && r.width % 4 == 0;
       if (r.width >= (1ull << 32) || r.rows >= (1ull << 32)) throw AdjError(TE_ERANGE, "undo-log region too large");
-      total += r.size();
-      cur += r.size();
+      total += B.vec[B.n] ? r.size() / 4 : r.size();
+      cur += r.logged();
+      acc.push_back(access_words(P.M + r.off, r.last() + 1 - r.off, restore));
       B.n++;
     }
     if (total >= (1ull << 32)) throw AdjError(TE_ERANGE, "undo-log regions of one op of 2^32 words or more");
     B.start[B.n] = (uint32_t)total;
     const int blocks = (int)std::min<uint64_t>(148 * 8, (total + 255) / 256);
-    launch_kernel(adj::k_batch_copy, dim3(blocks), dim3(256), 0, P.stream, P.M, log, B, restore ? 1 : 0);
-    ACU(cudaGetLastError());
+    in_order(deps, acc, [&] {
+      launch_kernel(adj::k_batch_copy, dim3(blocks), dim3(256), 0, P.stream, P.M, S.undo, (const uint64_t*)S.log_at, B,
+                    restore ? 1 : 0);
+    });
   }
 }
 
 // The undo-log words of one op's regions.
 uint64_t regions_words(const std::vector<Region>& regs) {
   uint64_t n = 0;
-  for (const Region& r : regs) n += r.size();
+  for (const Region& r : regs) n += r.logged();
   return n;
 }
 
-// Replays the active step op by op, saving each op's written regions at log + cursor.
-void logged_step(Plan& P, AdjointState& S, uint32_t* log) {
+// Replays the active step op by op, saving each op's written regions in the undo log.
+void logged_step(Plan& P, AdjointState& S, StepDeps* deps) {
   std::vector<Op>& ops = P.active->ops;
   uint64_t cur = 0;
   for (size_t i = 0; i < ops.size(); i++) {
@@ -608,66 +683,106 @@ void logged_step(Plan& P, AdjointState& S, uint32_t* log) {
       // intermediate state between them is never read (their adjoints read no values), so
       // every op's regions are saved before the run
       const AdjointState::HaloRun& R = S.runs[run];
-      copy_regions(P, R.regions, log, cur, false);
+      copy_regions(P, S, R.regions, cur, false, deps);
       cur += regions_words(R.regions);
-      launch_periodic_halos(ops[i].args.g, R.f, R.nf, P.stream);
-      ACU(cudaGetLastError());
+      std::vector<Access> acc;
+      for (int q = 0; q < R.nf; q++) acc.push_back(P.access(R.f[q], true));
+      in_order(deps, acc, [&] { launch_periodic_halos(ops[i].args.g, R.f, R.nf, P.stream); });
       i = (size_t)R.last;
       continue;
     }
-    copy_regions(P, S.regions[i], log, cur, false);
+    copy_regions(P, S, S.regions[i], cur, false, deps);
     cur += regions_words(S.regions[i]);
-    P.launch_exact(ops, (int)i, (int)i, false);
+    P.launch_exact(ops, (int)i, (int)i, false, deps);
   }
 }
 
 // Walks the active step's ops in reverse: restore the op's written regions, run its adjoint.
 // An op's regions are disjoint, except the x and y halo strips of one field in a halo run,
 // whose shared corner words were saved at the same moment and restore the same value.
-void reverse_step(Plan& P, AdjointState& S, const uint32_t* log) {
+void reverse_step(Plan& P, AdjointState& S, StepDeps* deps) {
   std::vector<Op>& ops = P.active->ops;
-  uint32_t* lg = const_cast<uint32_t*>(log);
   uint64_t cur = S.step_undo_words;
+  auto adjoint_of = [&](const float* f, bool add) {
+    const uint64_t off = (uint64_t)(reinterpret_cast<const uint32_t*>(f) - P.M);
+    Access a = access_words(S.L + off, P.region_len(off), !add);
+    a.add = add;
+    return a;
+  };
   for (size_t ii = ops.size(); ii-- > 0;) {
     const Op& o = ops[ii];
+    std::vector<Access> acc;
     if (S.run_to[ii] >= 0) {
       const AdjointState::HaloRun& R = S.runs[S.run_to[ii]];
       cur -= regions_words(R.regions);
-      copy_regions(P, R.regions, lg, cur, true);
-      adj::launch_adj_halo_run(R.adj, P.stream);
-      ACU(cudaGetLastError());
+      copy_regions(P, S, R.regions, cur, true, deps);
+      for (int q = 0; q < R.nf; q++) acc.push_back(adjoint_of(R.f[q], false));
+      in_order(deps, acc, [&] { adj::launch_adj_halo_run(R.adj, P.stream); });
       ii = (size_t)R.first;
       continue;
     }
     cur -= regions_words(S.regions[ii]);
-    copy_regions(P, S.regions[ii], lg, cur, true);
+    copy_regions(P, S, S.regions[ii], cur, true, deps);
     if (o.copy) {
       if ((o.n + 255) / 256 > 0x7fffffffu) throw AdjError(TE_ERANGE, "copy of 2^39 words or more");
-      launch_kernel(adj::k_adj_copy, dim3((unsigned)((o.n + 255) / 256)), dim3(256), 0, P.stream, S.L, o.src, o.dst,
-                    o.n);
+      acc = {access_words(S.L + o.src, o.n, true), access_words(S.L + o.dst, o.n, true)};
+      in_order(deps, acc, [&] {
+        launch_kernel(adj::k_adj_copy, dim3((unsigned)((o.n + 255) / 256)), dim3(256), 0, P.stream, S.L, o.src, o.dst,
+                      o.n);
+      });
     } else {
-      S.launch[ii](S.args[ii], P.stream);
+      const adj::AdjEntry* e = adj::find_adjoint(o.name);
+      for (int b = 0; b < kMaxBind; b++) {
+        if (!o.args.p[b]) continue;
+        if (e->reads >> b & 1u) acc.push_back(P.access(o.args.p[b], false));
+        if (e->owns >> b & 1u) acc.push_back(adjoint_of(o.args.p[b], false));
+        if (e->adds >> b & 1u) acc.push_back(adjoint_of(o.args.p[b], true));
+      }
+      in_order(deps, acc, [&] { S.launch[ii](S.args[ii], P.stream); });
     }
   }
 }
 
+// Launches the graph of `body` (logged_step or reverse_step) with the step's part of the undo
+// log at word `log`.  The two graphs serve every step of every block.  As in
+// Plan::launch_step_graph the concurrent form costs more to instantiate (8 ms of 440 nodes,
+// 1 ms as a chain) and is made once the chain has run kChainLaunches steps.  One B200, window
+// of 10 steps at 128x128x64 with its gradient: 84 -> 73 ms, its first pass 87 -> 81 ms (two
+// graphs where each of the K block positions had two).
+constexpr int kChainLaunches = 16;
+
 template <class F>
-cudaGraphExec_t capture(cudaStream_t s, F body) {
-  cudaGraph_t graph = nullptr;
-  ACU(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-  try {
-    body();
-  } catch (...) {
-    cudaStreamEndCapture(s, &graph);
-    if (graph) cudaGraphDestroy(graph);
-    throw;
+void launch_step(Plan& P, AdjointState& S, AdjointState::StepGraph& G, uint64_t log, F body) {
+  bool upgrade = G.launches >= kChainLaunches && !G.concurrent;
+  if (upgrade) {  // not while the caller captures the stream
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    ACU(cudaStreamIsCapturing(P.stream, &st));
+    upgrade = st == cudaStreamCaptureStatusNone;
   }
-  ACU(cudaStreamEndCapture(s, &graph));
-  cudaGraphExec_t ex = nullptr;
-  const cudaError_t e = cudaGraphInstantiate(&ex, graph, 0);
-  cudaGraphDestroy(graph);
-  ACU(e);
-  return ex;
+  if (!G.exec || upgrade) {
+    cudaGraph_t graph = nullptr;
+    ACU(cudaStreamBeginCapture(P.stream, cudaStreamCaptureModeThreadLocal));
+    try {
+      StepDeps deps(P.stream);
+      body(upgrade ? &deps : nullptr);
+      if (upgrade) ACU(deps.finish());
+    } catch (...) {
+      cudaStreamEndCapture(P.stream, &graph);
+      if (graph) cudaGraphDestroy(graph);
+      throw;
+    }
+    ACU(cudaStreamEndCapture(P.stream, &graph));
+    cudaGraphExec_t exec = nullptr;
+    const cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
+    cudaGraphDestroy(graph);
+    ACU(e);
+    G.chain = G.exec;
+    G.exec = exec;
+    G.concurrent = upgrade;
+  }
+  launch_kernel(adj::k_set_word, dim3(1), dim3(1), 0, P.stream, S.log_at, log);
+  ACU(cudaGraphLaunch(G.exec, P.stream));
+  if (G.launches < kChainLaunches) G.launches++;
 }
 
 int fail(te_ctx* ctx, int code, const std::string& m) {
@@ -713,10 +828,11 @@ int te_adjoint_forward(te_ctx* ctx, int nsteps, int checkpoint_every) {
     if (S.undo) cudaFree(S.undo);
     S.undo = nullptr;
     S.undo_cap = 0;
+    S.drop_graphs();  // they hold its address
     ACU(cudaMalloc(&S.undo, need * 4));
     S.undo_cap = need;
   }
-  if (S.every != checkpoint_every) S.drop_graphs();
+  if (!S.log_at) ACU(cudaMalloc(&S.log_at, sizeof(uint64_t)));
   S.every = checkpoint_every;
   S.nsteps = nsteps;
   for (int s = 0; s < nsteps; s++) {
@@ -738,27 +854,16 @@ int te_adjoint_backward(te_ctx* ctx) {
   te::build_tables(P, S);
   const int K = S.every;
   if ((uint64_t)K * S.step_undo_words > S.undo_cap) throw te::AdjError(TE_ESTATE, "step changed since te_adjoint_forward");
-  if ((int)S.fwd_graph.size() != K) {
-    S.drop_graphs();
-    S.fwd_graph.assign(K, nullptr);
-    S.rev_graph.assign(K, nullptr);
-  }
   const int nb = (S.nsteps + K - 1) / K;
   for (int b = nb - 1; b >= 0; b--) {
     const int s0 = b * K, s1 = std::min(s0 + K, S.nsteps);
     ACU(cudaMemcpyAsync(P.M, S.ckpt[b], S.ckpt_words * 4, cudaMemcpyDeviceToDevice, P.stream));
-    for (int s = s0; s < s1; s++) {
-      const int j = s - s0;
-      if (!S.fwd_graph[j])
-        S.fwd_graph[j] = te::capture(P.stream, [&] { te::logged_step(P, S, S.undo + (uint64_t)j * S.step_undo_words); });
-      ACU(cudaGraphLaunch(S.fwd_graph[j], P.stream));
-    }
-    for (int s = s1 - 1; s >= s0; s--) {
-      const int j = s - s0;
-      if (!S.rev_graph[j])
-        S.rev_graph[j] = te::capture(P.stream, [&] { te::reverse_step(P, S, S.undo + (uint64_t)j * S.step_undo_words); });
-      ACU(cudaGraphLaunch(S.rev_graph[j], P.stream));
-    }
+    for (int s = s0; s < s1; s++)
+      te::launch_step(P, S, S.fwd_graph, (uint64_t)(s - s0) * S.step_undo_words,
+                      [&](te::StepDeps* deps) { te::logged_step(P, S, deps); });
+    for (int s = s1 - 1; s >= s0; s--)
+      te::launch_step(P, S, S.rev_graph, (uint64_t)(s - s0) * S.step_undo_words,
+                      [&](te::StepDeps* deps) { te::reverse_step(P, S, deps); });
   }
   // fields that no adjoint operator reads are not logged: memory returns to the start
   // state from its checkpoint

@@ -24,15 +24,16 @@
 
 namespace te {
 
-// Device bytes [lo, hi) a launch reads or (write) may read and write.
+// Device bytes [lo, hi) a launch reads, or (write) may read and write, or (add) only adds to
+// with atomics: additions keep no order among themselves.
 struct Access {
   uintptr_t lo = 0, hi = 0;
-  bool write = false;
+  bool write = false, add = false;
 };
 
 inline Access access_words(const void* p, uint64_t words, bool write) {
   const uintptr_t a = reinterpret_cast<uintptr_t>(p);
-  return Access{a, a + words * 4, write};
+  return Access{a, a + words * 4, write, false};
 }
 
 class StepDeps {
@@ -52,7 +53,8 @@ class StepDeps {
       for (int q : ranges_[id].overlap) {
         const Range& r = ranges_[q];
         if (r.writer >= 0) after.push_back(r.writer);
-        if (a.write) after.insert(after.end(), r.readers.begin(), r.readers.end());
+        if (a.write || a.add) after.insert(after.end(), r.readers.begin(), r.readers.end());
+        if (!a.add) after.insert(after.end(), r.adders.begin(), r.adders.end());
       }
     }
     const int me = (int)tail_.size();
@@ -86,6 +88,9 @@ class StepDeps {
       if (a.write) {
         r.writer = me;
         r.readers.clear();
+        r.adders.clear();
+      } else if (a.add) {
+        r.adders.push_back(me);
       } else if (r.readers.empty() || r.readers.back() != me) {
         r.readers.push_back(me);
       }
@@ -110,6 +115,7 @@ class StepDeps {
     uintptr_t lo, hi;
     int writer = -1;           // the last launch that wrote (part of) it
     std::vector<int> readers;  // launches that read it since
+    std::vector<int> adders;   // launches that added to it since
     std::vector<int> overlap;  // the known ranges that share a byte with it, itself included
   };
 
