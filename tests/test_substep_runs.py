@@ -9,7 +9,11 @@ from thunderengine_web_b200 import scenario, timestep
 
 @pytest.mark.gpu
 @pytest.mark.parametrize('dims,nsound,align', [((5, 3, 8), 7, False), ((2, 9, 6), 8, False), ((33, 8, 5), 6, False),
-                                               ((64, 5, 13), 9, True), ((31, 40, 12), 2, False)])
+                                               ((64, 5, 13), 9, True), ((31, 40, 12), 2, False),
+                                               # the column kernel's sizes: 64 levels, 65 with one
+                                               # wave of tiles, 85
+                                               ((20, 9, 64), 4, False), ((33, 10, 65), 4, False),
+                                               ((16, 8, 85), 4, False)])
 def test_fused_steps_equal_the_oracle(dims, nsound, align):
     run = timestep.Run(scenario.tiny(*dims, dx=500.0, dz=250.0, dt=3.0, nsound=nsound, us=25.0, align_rows=align))
     tape = run.tape(1)

@@ -134,7 +134,7 @@ static void launch_acu_uv(const AcuArgs& A, cudaStream_t s) {
 // ------------------------------------------------------------ acoustic K2
 
 // K2: a CTA owns 32 interior columns (i0..i0+31, row j) and runs their implicit w-pi'
-// solve with warp specialisation.  kLevels worker warps (one level each per pass) load
+// solve with warp specialisation.  LEVELS worker warps (one level each per pass) load
 // the 19 inputs of their level, form fpk (acoustic_fpk.wgsl:167-207) and the tridiagonal
 // coefficients aa, bb, cc, dd of the level (lam_1, acoustic_w_solve.wgsl:124-139) into a
 // double-buffered pass store; the recurrence warp (one lane per column) runs the
@@ -149,36 +149,39 @@ static void launch_acu_uv(const AcuArgs& A, cudaStream_t s) {
 // per-dispatch kernels; sums the reference forms twice (pk1+qk, pp3d+fpk, ...) are formed
 // with the same rounding each time.
 //
-// Sized for three resident CTAs per SM (416 threads, 52 KB of shared memory at nz = 80):
-// more columns in flight hide the per-pass load latency better than a deeper pass.
-#ifndef TE_COL_LEVELS
-#define TE_COL_LEVELS 12   // worker warps = levels per pass
-#endif
-#ifndef TE_COL_MINB
-#define TE_COL_MINB 3      // resident CTAs per SM the register budget is sized for
-#endif
-#ifndef TE_COL_EPI
-#define TE_COL_EPI 7       // epilogue levels per worker per chunk
-#endif
+// Two sizes: 12 worker warps, three resident CTAs per SM (416 threads, 52 KB of shared memory
+// at nz = 80), and 8 workers, four CTAs, which hold 592 tiles at once instead of 444.  Up to
+// nz = 64 the smaller one is as fast or faster at every size measured (us, 8 against 12
+// workers, at nz = 60: 480 tiles 18.6 / 26.7, 800 28.8 / 30.9, 1280 51.3 / 50.8, 3040 104.6 /
+// 109.7; 505 tiles of 48 levels 14.5 / 22.7, 512 of 64 18.6 / 28.6).  Above that a wave of
+// smaller CTAs takes 1.3 times as long, and 1.8 times once four of them leave no L1 (nz > 84:
+// 900 tiles of 100 levels 89.5 / 75.8), so the waves decide (launch_acu_column): 2048 tiles of
+// 80 levels stay at 98.8 us with 12 workers (102.5 with 8).  Measured beside them at 505 /
+// 2048 tiles: 16 workers and two CTAs 20.6 us, 20 and two 26.8 us, 24 and one 32.9 us, 8 and
+// five (40 registers) 20.6 / 157 us, 4 and six 18.6 / 156 us.
 constexpr int kColTile = 32;
-constexpr int kLevels = TE_COL_LEVELS;
-constexpr int kWorkers = kColTile * kLevels;     // 384
-constexpr int kColThreads = kWorkers + kColTile; // + the recurrence warp
-constexpr int kEpiChunk = TE_COL_EPI;
+constexpr int kEpiChunk = 7;  // epilogue levels per worker per chunk (5: 102 us, 10: 112 us at 2048 tiles, 8 workers)
+template <int LEVELS>
+struct Col {
+  static constexpr int workers = kColTile * LEVELS;      // LEVELS worker warps = levels per pass
+  static constexpr int threads = workers + kColTile;     // + the recurrence warp
+  // [nz][32] cA, cB, s; [2][4][LEVELS][32] aa, bb, cc, dd per pass; [2][3][LEVELS][32] the
+  // exchange store (pk1 + qk, pk2 - qk, pi') per pass
+  static constexpr size_t smem(int nz) { return (size_t)(3 * nz + 14 * LEVELS) * kColTile * sizeof(float); }
+};
 
-// [nz][32] cA, cB, s; [2][4][kLevels][32] aa, bb, cc, dd per pass; [2][3][kLevels][32]
-// the exchange store (pk1 + qk, pk2 - qk, pi') per pass
-static size_t col_smem_bytes(int nz) { return (size_t)(3 * nz + 14 * kLevels) * kColTile * sizeof(float); }
-
+template <int LEVELS>
 __device__ __forceinline__ int co_at(int b, int term, int q, int lane) {
-  return ((b * 4 + term) * kLevels + q) * kColTile + lane;
+  return ((b * 4 + term) * LEVELS + q) * kColTile + lane;
 }
+template <int LEVELS>
 __device__ __forceinline__ int xs_at(int b, int term, int q, int lane) {
-  return ((b * 3 + term) * kLevels + q) * kColTile + lane;
+  return ((b * 3 + term) * LEVELS + q) * kColTile + lane;
 }
 
+template <int LEVELS>
 __device__ __forceinline__ void workers_sync() {
-  asm volatile("bar.sync 1, %0;" ::"n"(kWorkers) : "memory");
+  asm volatile("bar.sync 1, %0;" ::"n"(Col<LEVELS>::workers) : "memory");
 }
 // The CTA-wide barrier; workers and the recurrence warp reach it from separate code paths
 // (whole warps each), the same number of times.
@@ -227,30 +230,31 @@ __device__ __forceinline__ float fpk_of(const AcuArgs& A, const LevelIn& L, floa
   return fmaf(a.beta, fmaf(L.w0, L.pk1 + L.qk, L.w1 * (L.pk2 - L.qk)), fmaf(a.dts, fmaf(-L.ppterm, div, L.ppten), advPi));
 }
 
-// Forward recurrence over one pass of kLevels levels (acoustic_w_solve.wgsl:150-190): the
+// Forward recurrence over one pass of LEVELS levels (acoustic_w_solve.wgsl:150-190): the
 // coefficients of four levels are read from the pass store before the chain reaches them.
+template <int LEVELS>
 __device__ __forceinline__ void forward_pass(const float* co, float* cA, float* cB, int pp, int nz, int lane, float& cAm,
                                              float& cBm, float& wtop) {
-  const int b = pp & 1, base = pp * kLevels;
+  const int b = pp & 1, base = pp * LEVELS;
   float ca[4], cb[4], cc[4], cd[4];
 #pragma unroll
   for (int t = 0; t < 4; t++) {
-    ca[t] = co[co_at(b, 0, t, lane)];
-    cb[t] = co[co_at(b, 1, t, lane)];
-    cc[t] = co[co_at(b, 2, t, lane)];
-    cd[t] = co[co_at(b, 3, t, lane)];
+    ca[t] = co[co_at<LEVELS>(b, 0, t, lane)];
+    cb[t] = co[co_at<LEVELS>(b, 1, t, lane)];
+    cc[t] = co[co_at<LEVELS>(b, 2, t, lane)];
+    cd[t] = co[co_at<LEVELS>(b, 3, t, lane)];
   }
 #pragma unroll
-  for (int g4 = 0; g4 < kLevels / 4; g4++) {
+  for (int g4 = 0; g4 < LEVELS / 4; g4++) {
     float na[4], nb[4], nc[4], nd[4];
-    if (g4 + 1 < kLevels / 4) {
+    if (g4 + 1 < LEVELS / 4) {
 #pragma unroll
       for (int t = 0; t < 4; t++) {
         const int qq = 4 * (g4 + 1) + t;
-        na[t] = co[co_at(b, 0, qq, lane)];
-        nb[t] = co[co_at(b, 1, qq, lane)];
-        nc[t] = co[co_at(b, 2, qq, lane)];
-        nd[t] = co[co_at(b, 3, qq, lane)];
+        na[t] = co[co_at<LEVELS>(b, 0, qq, lane)];
+        nb[t] = co[co_at<LEVELS>(b, 1, qq, lane)];
+        nc[t] = co[co_at<LEVELS>(b, 2, qq, lane)];
+        nd[t] = co[co_at<LEVELS>(b, 3, qq, lane)];
       }
     }
     float oA[4], oB[4];
@@ -281,7 +285,7 @@ __device__ __forceinline__ void forward_pass(const float* co, float* cA, float* 
         cB[kk * kColTile + lane] = oB[t];
       }
     }
-    if (g4 + 1 < kLevels / 4) {
+    if (g4 + 1 < LEVELS / 4) {
 #pragma unroll
       for (int t = 0; t < 4; t++) {
         ca[t] = na[t];
@@ -324,15 +328,16 @@ __device__ __forceinline__ void back_substitute(float* cA, const float* cB, int 
   cA[lane] = 0.0f;
 }
 
-// The pi' update inputs of a worker's epilogue levels k0, k0 + kLevels, ...
+// The pi' update inputs of a worker's epilogue levels k0, k0 + LEVELS, ...
 struct EpiIn {
   float rr[kEpiChunk], pk1[kEpiChunk], qk[kEpiChunk], pk2[kEpiChunk], pp[kEpiChunk];
 };
 
+template <int LEVELS>
 __device__ __forceinline__ void load_epi(const AcuArgs& A, EpiIn& E, int c0, int k0, int nz, int sk) {
 #pragma unroll
   for (int t = 0; t < kEpiChunk; t++) {
-    const int k = k0 + t * kLevels;
+    const int k = k0 + t * LEVELS;
     if (k <= nz) {
       const int c = c0 + k * sk;
       E.rr[t] = A.rrw[c];
@@ -346,7 +351,8 @@ __device__ __forceinline__ void load_epi(const AcuArgs& A, EpiIn& E, int c0, int
   }
 }
 
-__global__ void __launch_bounds__(kColThreads, TE_COL_MINB) k_acu_column(AcuArgs A) {
+template <int LEVELS, int MINB>
+__global__ void __launch_bounds__(Col<LEVELS>::threads, MINB) k_acu_column(AcuArgs A) {
   extern __shared__ float smem[];
   const Dims& g = A.g;
   const Acoustic& a = A.a;
@@ -355,24 +361,24 @@ __global__ void __launch_bounds__(kColThreads, TE_COL_MINB) k_acu_column(AcuArgs
   float* cB = smem + nz * kColTile;
   float* sS = smem + 2 * nz * kColTile;
   float* co = smem + 3 * nz * kColTile;
-  float* xs = co + 8 * kLevels * kColTile;
+  float* xs = co + 8 * LEVELS * kColTile;
   const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
   const int i = blockIdx.x * kColTile + lane;
   const int j = blockIdx.y;
   const bool col = i < g.nx;
   const int sk = g.sJ * g.sK;
   const int c0 = gidx(g, col ? i : 0, j, 0);
-  const int npass = (nz + kLevels - 1) / kLevels;
-  if (q == kLevels) {
+  const int npass = (nz + LEVELS - 1) / LEVELS;
+  if (q == LEVELS) {
     // recurrence warp: pass p - 1 while the workers prepare pass p, then the last pass
     // and the back substitution
     float cAm = 0.0f, cBm = 0.0f, wtop = 0.0f;
     for (int p = 0; p < npass; p++) {
-      if (p >= 1 && col) forward_pass(co, cA, cB, p - 1, nz, lane, cAm, cBm, wtop);
+      if (p >= 1 && col) forward_pass<LEVELS>(co, cA, cB, p - 1, nz, lane, cAm, cBm, wtop);
       block_sync();
     }
     if (col) {
-      forward_pass(co, cA, cB, npass - 1, nz, lane, cAm, cBm, wtop);
+      forward_pass<LEVELS>(co, cA, cB, npass - 1, nz, lane, cAm, cBm, wtop);
       back_substitute(cA, cB, nz, lane, wtop);
     }
     block_sync();
@@ -381,7 +387,7 @@ __global__ void __launch_bounds__(kColThreads, TE_COL_MINB) k_acu_column(AcuArgs
   const float asq = a.alph * a.alph;
   const float uh = hm_uh(g, A.hm, col ? i : 0), vh = hm_vh(g, A.hm, j);
   for (int p = 0; p < npass; p++) {
-    const int k = p * kLevels + q;
+    const int k = p * LEVELS + q;
     const bool ok = col && k < nz;
     const int b = p & 1;
     float m = 0.0f, wt = 0.0f, w0 = 0.0f, vA = 0.0f, vB = 0.0f, vP = 0.0f, vS = 0.0f;
@@ -393,39 +399,39 @@ __global__ void __launch_bounds__(kColThreads, TE_COL_MINB) k_acu_column(AcuArgs
       vP = cur.pp;
       vS = cur.pp + fk;
       sS[k * kColTile + lane] = vS;
-      xs[xs_at(b, 0, q, lane)] = vA;
-      xs[xs_at(b, 1, q, lane)] = vB;
-      xs[xs_at(b, 2, q, lane)] = vP;
+      xs[xs_at<LEVELS>(b, 0, q, lane)] = vA;
+      xs[xs_at<LEVELS>(b, 1, q, lane)] = vB;
+      xs[xs_at<LEVELS>(b, 2, q, lane)] = vP;
       m = cur.mm;
       wt = cur.wt;
       w0 = cur.w0;
     }
-    workers_sync();
+    workers_sync<LEVELS>();
     if (ok && k >= 1) {
       // level k - 1: the previous warp of this pass, or the last warp of the previous one
-      const int bp = q > 0 ? b : b ^ 1, qp = q > 0 ? q - 1 : kLevels - 1;
-      const float pA = xs[xs_at(bp, 0, qp, lane)], pB = xs[xs_at(bp, 1, qp, lane)], pP = xs[xs_at(bp, 2, qp, lane)];
+      const int bp = q > 0 ? b : b ^ 1, qp = q > 0 ? q - 1 : LEVELS - 1;
+      const float pA = xs[xs_at<LEVELS>(bp, 0, qp, lane)], pB = xs[xs_at<LEVELS>(bp, 1, qp, lane)], pP = xs[xs_at<LEVELS>(bp, 2, qp, lane)];
       const float pS = sS[(k - 1) * kColTile + lane];
-      co[co_at(b, 0, q, lane)] = (-asq) * (m * pA);
-      co[co_at(b, 2, q, lane)] = (-asq) * ((-m) * vB);
-      co[co_at(b, 1, q, lane)] = fmaf(-asq, m * ((-vA) + pB), 1.0f);
+      co[co_at<LEVELS>(b, 0, q, lane)] = (-asq) * (m * pA);
+      co[co_at<LEVELS>(b, 2, q, lane)] = (-asq) * ((-m) * vB);
+      co[co_at<LEVELS>(b, 1, q, lane)] = fmaf(-asq, m * ((-vA) + pB), 1.0f);
       const float fw = fmaf(a.dts, wt, a.beta * ((-m) * (vP - pP)));
-      co[co_at(b, 3, q, lane)] = fmaf(a.alph, (-m) * (vS - pS), w0 + fw);
+      co[co_at<LEVELS>(b, 3, q, lane)] = fmaf(a.alph, (-m) * (vS - pS), w0 + fw);
     }
     block_sync();
   }
   // the epilogue's first loads fly during the last forward pass and the back substitution
   EpiIn E;
-  if (col) load_epi(A, E, c0, q, nz, sk);
+  if (col) load_epi<LEVELS>(A, E, c0, q, nz, sk);
   block_sync();
   if (!col) return;
-  // pi' update and stores, levels q, q + kLevels, ... (acoustic_pp.wgsl:131-167,
+  // pi' update and stores, levels q, q + LEVELS, ... (acoustic_pp.wgsl:131-167,
   // acoustic_accumulate.wgsl:129-158)
-  for (int k0 = q; k0 <= nz; k0 += kEpiChunk * kLevels) {
-    if (k0 != q) load_epi(A, E, c0, k0, nz, sk);
+  for (int k0 = q; k0 <= nz; k0 += kEpiChunk * LEVELS) {
+    if (k0 != q) load_epi<LEVELS>(A, E, c0, k0, nz, sk);
 #pragma unroll
     for (int t = 0; t < kEpiChunk; t++) {
-      const int k = k0 + t * kLevels;
+      const int k = k0 + t * LEVELS;
       if (k > nz) break;
       const int c = c0 + k * sk;
       if (k < nz) {
@@ -449,11 +455,26 @@ __global__ void __launch_bounds__(kColThreads, TE_COL_MINB) k_acu_column(AcuArgs
   }
 }
 
+template <int LEVELS, int MINB>
+static int col_resident(int nz) {  // CTAs of the GPU's 148 SMs, 227 KB of shared memory each
+  return 148 * std::max(1, std::min<int>(MINB, (int)(227 * 1024 / (Col<LEVELS>::smem(nz) + 1024))));
+}
+
+template <int LEVELS, int MINB>
+static void launch_acu_column_t(const AcuArgs& A, cudaStream_t s) {
+  const size_t bytes = Col<LEVELS>::smem(A.g.nz);
+  if (opt_in_smem((const void*)k_acu_column<LEVELS, MINB>, bytes) != cudaSuccess) return;  // error left pending
+  dim3 b(Col<LEVELS>::threads), gr((A.g.nx + kColTile - 1) / kColTile, A.g.ny);
+  launch_kernel(k_acu_column<LEVELS, MINB>, dim3(gr), dim3(b), bytes, s, A);
+}
+
 static void launch_acu_column(const AcuArgs& A, cudaStream_t s) {
-  const size_t bytes = col_smem_bytes(A.g.nz);
-  if (opt_in_smem((const void*)k_acu_column, bytes) != cudaSuccess) return;  // error left pending
-  dim3 b(kColThreads), gr((A.g.nx + kColTile - 1) / kColTile, A.g.ny);
-  launch_kernel(k_acu_column, dim3(gr), dim3(b), bytes, s, A);
+  const long tiles = (long)((A.g.nx + kColTile - 1) / kColTile) * A.g.ny;
+  const long r12 = col_resident<12, 3>(A.g.nz), r8 = col_resident<8, 4>(A.g.nz);
+  const long w12 = (tiles + r12 - 1) / r12, w8 = (tiles + r8 - 1) / r8;
+  const long wave8 = A.g.nz <= 84 ? 13 : 18;  // time of a wave of 8-worker CTAs, tenths of a 12-worker one's
+  if (A.g.nz <= 64 || wave8 * w8 < 10 * w12) launch_acu_column_t<8, 4>(A, s);
+  else launch_acu_column_t<12, 3>(A, s);
 }
 
 // ------------------------------------------------------------ periodic halos
@@ -1025,7 +1046,7 @@ static bool match_substep(const std::vector<Op>& ops, size_t i, FusedSegment& s,
   const Op& acc = ops[i + 6];
   if (!is_name(acc, "acoustic_accumulate")) return false;
   const Dims& g = uv.args.g;
-  if (g.nx < 1 || g.ny < 1 || g.nz < 3 || col_smem_bytes(g.nz) > 200 * 1024)
+  if (g.nx < 1 || g.ny < 1 || g.nz < 3 || Col<12>::smem(g.nz) > 200 * 1024)
     return false;
   for (const Op* o : {&fp, &ws, &pp, &acc})
     if (!same_dims(g, o->args.g) || !same_acoustic(uv.args.a, o->args.a)) return false;
