@@ -2378,22 +2378,42 @@ __global__ void k_morr_prep(KArgs A) {
 }
 TE_LAUNCH3(morr_prep)
 
-// morr_column.wgsl: one thread per column (te_morr.cuh morr::column), the dispatch's rows
-// taken scr_rows at a time (the reference's y tiles: the planned per-thread scratch holds
-// that many rows); each launch lays the scratch out by array, level, then column of the
-// tile, so the threads of a warp touch consecutive words.
-__global__ void __launch_bounds__(128) k_morr_column(KArgs A, int y0, int rows) {
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int ncol = A.gx * rows;
-  if (t >= ncol) return;
-  const int i = t % A.gx, j = y0 + t / A.gx;
-  if (j >= A.gy) return;
-  morr::Params p;
+// morr_column.wgsl (te_morr.cuh): a block per 32 columns, its warps on the levels.  The process
+// rates, fall speeds and updates of a level depend on no other level; a sedimentation substep
+// takes every level's flux from the state before it, so it too runs level-parallel, the fluxes
+// exchanged through shared memory between two barriers.  What stays in the reference's order
+// per column: the speeds handed down to levels without any, and the precipitation sum.
+//
+// One thread per column, the reference's form, had 450 warps for 120 x 120 columns, each
+// walking 40 levels of pow and exp evaluations, and was bound by one warp's latency.  One B200,
+// per launch, thread per column -> this, after 2 / 60 / 140 steps of the recorded storms:
+// 120x120x40 127 / 600 / 961 -> 66 / 104 / 149 us, 300x60x40 132 / 784 / 1214 -> 69 / 162 /
+// 221 us.  8 warps a block 55 / 127 / 177 us, 4 warps 56 / 197 / 283 us on the first.
+//
+// The dispatch's rows are taken scr_rows at a time (the reference's y tiles: the planned
+// per-thread scratch holds that many rows); each launch lays the scratch out by array,
+// level, then column of the tile, so the lanes of a warp touch consecutive words.
+constexpr int kMorrCols = 32;
+constexpr int kMorrWarps = 16;
+
+static size_t morr_smem(int nz) { return (size_t)8 * nz * kMorrCols * sizeof(float); }
+
+__global__ void __launch_bounds__(kMorrCols* kMorrWarps) k_morr_column(KArgs A, int y0, int rows) {
+  extern __shared__ float msm[];
+  __shared__ morr::Params p;
+  __shared__ int steps[kMorrCols], active[kMorrCols];
+  const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
   {
     uint32_t* w = reinterpret_cast<uint32_t*>(&p);
-    for (int q = 0; q < (int)(sizeof(morr::Params) / 4); q++) w[q] = A.ref0[q];
+    for (int q = threadIdx.x; q < (int)(sizeof(morr::Params) / 4); q += blockDim.x) w[q] = A.ref0[q];
+    if (wq == 0) active[lane] = 0;
   }
-  if (i >= p.nx || j >= p.ny) return;
+  __syncthreads();
+  const int t = blockIdx.x * kMorrCols + lane, ncol = A.gx * rows;
+  const int i = t % A.gx, j = y0 + t / A.gx;
+  const bool col = t < ncol && j < A.gy && i < p.nx && j < p.ny;
+  const int nk = p.nz, dorad = A.iv[19];
+  const float DT = p.dt;
   morr::Fields F;
   F.T3 = A.p[1];
   F.QV = A.p[2];
@@ -2413,41 +2433,135 @@ __global__ void __launch_bounds__(128) k_morr_column(KArgs A, int y0, int rows) 
   F.EFFC = A.p[16];
   F.EFFI = A.p[17];
   F.EFFS = A.p[18];
-  const morr::Scratch S{A.scr + t, (unsigned)ncol, p.nz};
-  morr::column(p, F, S, i, j, A.iv[19]);
+  const morr::Scratch S{A.scr + (col ? t : 0), (unsigned)ncol, nk};
+  if (col) {
+    bool act = false;
+    for (int k = wq; k < nk; k += kMorrWarps) act = morr::level_rates(p, F, S, i, j, k, dorad) || act;
+    if (act) active[lane] = 1;
+  }
+  __syncthreads();
+  const bool on = col && active[lane] != 0;
+  if (!__syncthreads_or(on)) return;
+  // per level and column: speeds (mass, number), contents, fluxes, tendencies
+  const int row = nk * kMorrCols;
+  float *sU = msm + lane, *sN = sU + row, *sQ = sN + row, *sC = sQ + row, *sFq = sC + row, *sFn = sFq + row;
+  float *sTq = sFn + row, *sTn = sTq + row;
+  float precrt = 0.0f;
+  for (int s = 0; s < 5; s++) {
+    const int ntend = morr::number_tendency(s);
+    if (wq == 0) steps[lane] = 1;
+    if (on)
+      for (int k = wq; k < nk; k += kMorrWarps) {
+        const int e = k * kMorrCols;
+        morr::fall_speed(p, F, S, s, i, j, k, sU[e], sN[e], sQ[e], sC[e]);
+        sTq[e] = S(2304 + s * 128, k);
+        sTn[e] = S(ntend, k);
+      }
+    __syncthreads();
+    if (on && wq < 2) {
+      float* a = wq == 0 ? sU : sN;
+      float above = a[(nk - 1) * kMorrCols];
+      for (int k = nk - 2; k >= 0; k--) {
+        float v = a[k * kMorrCols];
+        if (v < 1e-10f) {
+          v = above;
+          a[k * kMorrCols] = v;
+        }
+        above = v;
+      }
+    }
+    __syncthreads();
+    if (on)
+      for (int k = wq; k < nk; k += kMorrWarps) {
+        const float rgvm = morr_max(sU[k * kMorrCols], sN[k * kMorrCols]);
+        atomicMax(&steps[lane], (int)fmaf(rgvm * DT, morr_div(1.0f, F.DZQ[k]), 1.0f));
+      }
+    __syncthreads();
+    const int nstep = on ? steps[lane] : 0;
+    const int most = __reduce_max_sync(0xffffffffu, nstep);  // every warp has the same columns
+    const float dttmp = morr_div(DT, (float)nstep);
+    for (int n = 0; n < most; n++) {
+      const bool fall = n < nstep;
+      if (fall)
+        for (int k = wq; k < nk; k += kMorrWarps) {
+          const int e = k * kMorrCols;
+          sFq[e] = sU[e] * sQ[e];
+          sFn[e] = sN[e] * sC[e];
+        }
+      __syncthreads();
+      if (fall) {
+        for (int k = wq; k < nk; k += kMorrWarps) {
+          const int e = k * kMorrCols;
+          const float temr = morr_div(1.0f, (float)nstep * F.RH3[morr::mi(p, i, j, k)]);
+          const float temz = morr_div(1.0f, F.DZQ[k]);
+          // the top level loses its flux, the others gain the difference to the level above
+          float fq, fn;
+          if (k == nk - 1) {
+            fq = -(sFq[e] * temz);
+            fn = -(sFn[e] * temz);
+          } else {
+            fq = (sFq[e + kMorrCols] - sFq[e]) * temz;
+            fn = (sFn[e + kMorrCols] - sFn[e]) * temz;
+          }
+          sTq[e] = fmaf(fq, temr, sTq[e]);
+          sTn[e] = fmaf(fn, temr, sTn[e]);
+          sQ[e] = fmaf(fq, dttmp, sQ[e]);
+          sC[e] = fmaf(fn, dttmp, sC[e]);
+        }
+        if (wq == 0) precrt = fmaf(sFq[0], dttmp, precrt);
+      }
+      __syncthreads();
+    }
+    if (on)
+      for (int k = wq; k < nk; k += kMorrWarps) {
+        S(2304 + s * 128, k) = sTq[k * kMorrCols];
+        S(ntend, k) = sTn[k * kMorrCols];
+      }
+    __syncthreads();  // steps and the arrays are the next species'
+  }
+  if (!on) return;
+  for (int k = wq; k < nk; k += kMorrWarps) morr::level_update(p, F, S, i, j, k, dorad);
+  if (wq == 0) {
+    const int c0 = morr::mi(p, i, j, 0);
+    F.sfc[c0] = F.sfc[c0] + precrt;
+  }
 }
 
 // (nz <= 128 and a one-level dispatch grid are checked at plan time, Plan::finalize_args)
 static void launch_morr_column(const KArgs& A, cudaStream_t s) {
   const int rows = A.scr_rows > 0 ? (int)A.scr_rows : A.gy;
+  const size_t bytes = morr_smem(A.g.nz);
+  if (opt_in_smem((const void*)k_morr_column, bytes) != cudaSuccess) return;  // error left pending
   for (int y0 = 0; y0 < A.gy; y0 += rows) {
     const int r = std::min(rows, A.gy - y0);
     const int ncol = A.gx * r;
-    launch_kernel(k_morr_column, dim3((ncol + 127) / 128), dim3(128), 0, s, A, y0, r);
+    launch_kernel(k_morr_column, dim3((ncol + kMorrCols - 1) / kMorrCols), dim3(kMorrCols * kMorrWarps), bytes, s, A, y0, r);
   }
 }
 
-// morr_refl10cm.wgsl: one thread per column (te_refl.cuh morr::refl_column), the
-// dispatch's rows taken scr_rows at a time like morr_column, the 11 per-level arrays in the
-// planned scratch laid out by array, level, then column of the tile.
-__global__ void __launch_bounds__(128) k_morr_refl10cm(KArgs A, int y0, int rows) {
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int ncol = A.gx * rows;
-  if (t >= ncol) return;
-  const int i = t % A.gx, j = y0 + t / A.gx;
-  if (j >= A.gy) return;
-  morr::Params p;
+// morr_refl10cm.wgsl (te_refl.cuh), blocks and tiles as morr_column: a level's reflectivities and
+// its melting-particle integral depend on the column only through the level the melting
+// layer starts at.  One B200, per launch, thread per column -> this: 120x120x40 173-189 -> 71-84
+// us, 300x60x40 177 -> 79 us (storms without and with condensate).
+constexpr int kReflWarps = 8;
+
+__global__ void __launch_bounds__(kMorrCols* kReflWarps) k_morr_refl10cm(KArgs A, int y0, int rows) {
+  __shared__ morr::Params p;
+  __shared__ morr::RadarHead h;
+  __shared__ int top[kMorrCols];
+  const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
   {
     uint32_t* w = reinterpret_cast<uint32_t*>(&p);
-    for (int q = 0; q < (int)(sizeof(morr::Params) / 4); q++) w[q] = A.ref0[q];
-  }
-  if (i >= p.nx || j >= p.ny) return;
-  morr::RadarHead h;
-  {
+    for (int q = threadIdx.x; q < (int)(sizeof(morr::Params) / 4); q += blockDim.x) w[q] = A.ref0[q];
     const uint32_t* src = reinterpret_cast<const uint32_t*>(A.p[1]);
-    uint32_t* w = reinterpret_cast<uint32_t*>(&h);
-    for (int q = 0; q < (int)(sizeof(morr::RadarHead) / 4); q++) w[q] = src[q];
+    w = reinterpret_cast<uint32_t*>(&h);
+    for (int q = threadIdx.x; q < (int)(sizeof(morr::RadarHead) / 4); q += blockDim.x) w[q] = src[q];
   }
+  __syncthreads();
+  const int t = blockIdx.x * kMorrCols + lane, ncol = A.gx * rows;
+  const int i = t % A.gx, j = y0 + t / A.gx;
+  const bool col = t < ncol && j < A.gy && i < p.nx && j < p.ny;
+  const int nk = p.nz;
   morr::RadarFields F;
   F.bs = A.p[2];
   F.bg = A.p[3];
@@ -2461,18 +2575,25 @@ __global__ void __launch_bounds__(128) k_morr_refl10cm(KArgs A, int y0, int rows
   F.NG = A.p[11];
   F.RH = A.p[12];
   F.dbz = A.p[13];
-  const morr::Scratch S{A.scr + t, (unsigned)ncol, p.nz};
-  morr::refl_column(p, h, F, S, i, j);
+  const morr::Scratch S{A.scr + (col ? t : 0), (unsigned)ncol, nk};
+  if (col)
+    for (int k = wq; k < nk; k += kReflWarps) morr::refl_level(p, h, F, S, i, j, k);
+  __syncthreads();
+  if (col && wq == 0) top[lane] = morr::refl_melting_top(S, nk);
+  __syncthreads();
+  if (!col) return;
+  for (int k = wq; k < nk; k += kReflWarps) {
+    if (k < top[lane]) morr::refl_melting(h, F, S, k, top[lane]);
+    morr::refl_dbz(p, F, S, i, j, k);
+  }
 }
 
-// (nz <= 128, a one-level dispatch grid and bound head, bins and weights are checked at
-// plan time, Plan::finalize_args)
 static void launch_morr_refl10cm(const KArgs& A, cudaStream_t s) {
   const int rows = A.scr_rows > 0 ? (int)A.scr_rows : A.gy;
   for (int y0 = 0; y0 < A.gy; y0 += rows) {
     const int r = std::min(rows, A.gy - y0);
     const int ncol = A.gx * r;
-    launch_kernel(k_morr_refl10cm, dim3((ncol + 127) / 128), dim3(128), 0, s, A, y0, r);
+    launch_kernel(k_morr_refl10cm, dim3((ncol + kMorrCols - 1) / kMorrCols), dim3(kMorrCols * kReflWarps), 0, s, A, y0, r);
   }
 }
 

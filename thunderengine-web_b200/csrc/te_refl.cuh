@@ -152,85 +152,92 @@ TE_MORR_HD float pow7(float s) {
   return (s4 * s2) * s;
 }
 
-// main of morr_refl10cm.wgsl (:464-657) for column (i, j): the Rayleigh reflectivities
-// of rain, snow and graupel per level (Z = 720 n0 / lambda^7), in a melting layer (below
-// the lowest level k0 over rain above 0 C with snow and graupel above it) the snow and
-// graupel terms replaced by the melting-particle integral over 100 bins, then
-// dbz = 10 log10((Zr + Zs + Zg) 1e18).
+// The per-level arrays of main of morr_refl10cm.wgsl (:464-657).
+enum { kQr = 0, kQs = 128, kQg = 256, kT = 384, kIls = 512, kN0s = 640, kIlg = 768, kN0g = 896, kZr = 1024,
+       kZs = 1152, kZg = 1280 };
+constexpr float kReflR1 = 1e-12f;
+
+// The Rayleigh reflectivities of rain, snow and graupel at level k (Z = 720 n0 / lambda^7).
+TE_MORR_HD void refl_level(const Params& p, const RadarHead& h, const RadarFields& F, const Scratch& S, int i, int j, int k) {
+  const float R1 = kReflR1;
+  const int c = mi(p, i, j, k);
+  const float rho = F.RH[c];
+  S(kT, k) = F.T[c];
+  const float qr = F.QR[c], qs = F.QS[c], qg = F.QG[c], nr = F.NR[c], ns = F.NS[c], ng = F.NG[c];
+  const bool lr = qr > R1, ls = qs > R1, lg = qg > R1;
+  const float rqr = lr ? qr * rho : R1, rqs = ls ? qs * rho : R1, rqg = lg ? qg * rho : R1;
+  S(kQr, k) = rqr;
+  S(kQs, k) = rqs;
+  S(kQg, k) = rqg;
+  const float rnr = nr > R1 ? nr * rho : R1, rns = ns > R1 ? ns * rho : R1, rng = ng > R1 ? ng * rho : R1;
+  float lam, n0;
+  slope(p.cons[1], rns, rqs, rho, p.lammins, p.lammaxs, lam, n0);
+  const float ils = morr_div(1.0f, lam), n0s = n0;
+  S(kIls, k) = ils;
+  S(kN0s, k) = n0s;
+  slope(p.cons[2], rng, rqg, rho, p.lamming, p.lammaxg, lam, n0);
+  const float ilg = morr_div(1.0f, lam), n0g = n0;
+  S(kIlg, k) = ilg;
+  S(kN0g, k) = n0g;
+  slope(p.pi * p.rhow, rnr, rqr, rho, p.lamminr, p.lammaxr, lam, n0);
+  S(kZr, k) = lr ? (n0 * 720.0f) * pow7(morr_div(1.0f, lam)) : 1e-22f;
+  S(kZs, k) = ls ? ((h.zfac_s * n0s) * 720.0f) * pow7(ils) : 1e-22f;
+  S(kZg, k) = lg ? ((h.zfac_g * n0g) * 720.0f) * pow7(ilg) : 1e-22f;
+}
+
+// The level above the melting layer: the first level from the top with rain above 0 C under
+// snow or graupel, plus one; 0 where there is none.
+TE_MORR_HD int refl_melting_top(const Scratch& S, int nk) {
+  const float T_0 = 273.15f;
+  for (int k = nk - 2; k >= 0; k--)
+    if (S(kT, k) > T_0 && S(kQr, k) > 1e-06f && S(kQs, k + 1) + S(kQg, k + 1) > 1e-05f) return k + 1;
+  return 0;
+}
+
+// Level k < k0 of the melting layer below level k0: its snow and graupel terms replaced by the
+// melting-particle integral over 100 bins.
+TE_MORR_HD void refl_melting(const RadarHead& h, const RadarFields& F, const Scratch& S, int k, int k0) {
+  const float R1 = kReflR1, kfac = morr_div(h.lamda4, h.pi5 * h.kw);
+  const float fs = morr_min(1.0f - morr_div(S(kQs, k), S(kQs, k0)), 1.0f);
+  if (fs > 0.01f && fs < 0.99f && S(kQs, k) > R1) {
+    const float n0s = S(kN0s, k), ils = S(kIls, k);
+    float eta = 0.0f;
+    for (int n = 0; n < kBins; n++) {
+      const float* b = F.bs + n * kBinWords;
+      const float cb = soak(h, b, fs);
+      const float fd = n0s * morr_exp(morr_div(-b[kBinD], ils));
+      eta = fmaf((fd * cb) * F.simpson[n], b[kBinDt], eta);
+    }
+    S(kZs, k) = kfac * eta;
+  }
+  const float fg = morr_min(1.0f - morr_div(S(kQg, k), S(kQg, k0)), 1.0f);
+  if (fg > 0.01f && fg < 0.99f && S(kQg, k) > R1) {
+    const float n0g = S(kN0g, k), lamg = morr_div(1.0f, S(kIlg, k));
+    float eta = 0.0f;
+    for (int n = 0; n < kBins; n++) {
+      const float* b = F.bg + n * kBinWords;
+      const float cb = soak(h, b, fg);
+      const float fd = n0g * morr_exp((-lamg) * b[kBinD]);
+      eta = fmaf((fd * cb) * F.simpson[n], b[kBinDt], eta);
+    }
+    S(kZg, k) = kfac * eta;
+  }
+}
+
+TE_MORR_HD void refl_dbz(const Params& p, const RadarFields& F, const Scratch& S, int i, int j, int k) {
+  const float z = (S(kZr, k) + S(kZs, k)) + S(kZg, k);
+  F.dbz[mi(p, i, j, k)] = 10.0f * (morr_log2(z * 1e+18f) * 0.30103f);
+}
+
+// main of morr_refl10cm.wgsl (:464-657) for column (i, j), in its order: the reflectivities per
+// level, in a melting layer the integrals, then dbz = 10 log10((Zr + Zs + Zg) 1e18).  (The
+// CUDA kernel runs the levels of a column in parallel; this is the serial form.)
 TE_MORR_HD void refl_column(const Params& p, const RadarHead& h, const RadarFields& F, const Scratch& S, int i, int j) {
   const int nk = p.nz;
-  const float R1 = 1e-12f, T_0 = 273.15f;
-  enum { kQr = 0, kQs = 128, kQg = 256, kT = 384, kIls = 512, kN0s = 640, kIlg = 768, kN0g = 896, kZr = 1024,
-         kZs = 1152, kZg = 1280 };
-  for (int k = 0; k < nk; k++) {
-    const int c = mi(p, i, j, k);
-    const float rho = F.RH[c];
-    S(kT, k) = F.T[c];
-    const float qr = F.QR[c], qs = F.QS[c], qg = F.QG[c], nr = F.NR[c], ns = F.NS[c], ng = F.NG[c];
-    const bool lr = qr > R1, ls = qs > R1, lg = qg > R1;
-    const float rqr = lr ? qr * rho : R1, rqs = ls ? qs * rho : R1, rqg = lg ? qg * rho : R1;
-    S(kQr, k) = rqr;
-    S(kQs, k) = rqs;
-    S(kQg, k) = rqg;
-    const float rnr = nr > R1 ? nr * rho : R1, rns = ns > R1 ? ns * rho : R1, rng = ng > R1 ? ng * rho : R1;
-    float lam, n0;
-    slope(p.cons[1], rns, rqs, rho, p.lammins, p.lammaxs, lam, n0);
-    const float ils = morr_div(1.0f, lam), n0s = n0;
-    S(kIls, k) = ils;
-    S(kN0s, k) = n0s;
-    slope(p.cons[2], rng, rqg, rho, p.lamming, p.lammaxg, lam, n0);
-    const float ilg = morr_div(1.0f, lam), n0g = n0;
-    S(kIlg, k) = ilg;
-    S(kN0g, k) = n0g;
-    slope(p.pi * p.rhow, rnr, rqr, rho, p.lamminr, p.lammaxr, lam, n0);
-    S(kZr, k) = lr ? (n0 * 720.0f) * pow7(morr_div(1.0f, lam)) : 1e-22f;
-    S(kZs, k) = ls ? ((h.zfac_s * n0s) * 720.0f) * pow7(ils) : 1e-22f;
-    S(kZg, k) = lg ? ((h.zfac_g * n0g) * 720.0f) * pow7(ilg) : 1e-22f;
-  }
-  // the melting layer: the first level from the top with rain above 0 C under snow or
-  // graupel
-  int k0 = 0;
-  bool melti = false;
-  for (int k = nk - 2; k >= 0; k--) {
-    if (S(kT, k) > T_0 && S(kQr, k) > 1e-06f && S(kQs, k + 1) + S(kQg, k + 1) > 1e-05f) {
-      k0 = k + 1 > k0 ? k + 1 : k0;
-      melti = true;
-      break;
-    }
-  }
-  if (melti && k0 >= 1) {
-    const float kfac = morr_div(h.lamda4, h.pi5 * h.kw);
-    for (int k = k0 - 1; k >= 0; k--) {
-      const float fs = morr_min(1.0f - morr_div(S(kQs, k), S(kQs, k0)), 1.0f);
-      if (fs > 0.01f && fs < 0.99f && S(kQs, k) > R1) {
-        const float n0s = S(kN0s, k), ils = S(kIls, k);
-        float eta = 0.0f;
-        for (int n = 0; n < kBins; n++) {
-          const float* b = F.bs + n * kBinWords;
-          const float cb = soak(h, b, fs);
-          const float fd = n0s * morr_exp(morr_div(-b[kBinD], ils));
-          eta = fmaf((fd * cb) * F.simpson[n], b[kBinDt], eta);
-        }
-        S(kZs, k) = kfac * eta;
-      }
-      const float fg = morr_min(1.0f - morr_div(S(kQg, k), S(kQg, k0)), 1.0f);
-      if (fg > 0.01f && fg < 0.99f && S(kQg, k) > R1) {
-        const float n0g = S(kN0g, k), lamg = morr_div(1.0f, S(kIlg, k));
-        float eta = 0.0f;
-        for (int n = 0; n < kBins; n++) {
-          const float* b = F.bg + n * kBinWords;
-          const float cb = soak(h, b, fg);
-          const float fd = n0g * morr_exp((-lamg) * b[kBinD]);
-          eta = fmaf((fd * cb) * F.simpson[n], b[kBinDt], eta);
-        }
-        S(kZg, k) = kfac * eta;
-      }
-    }
-  }
-  for (int k = 0; k < nk; k++) {
-    const float z = (S(kZr, k) + S(kZs, k)) + S(kZg, k);
-    F.dbz[mi(p, i, j, k)] = 10.0f * (morr_log2(z * 1e+18f) * 0.30103f);
-  }
+  for (int k = 0; k < nk; k++) refl_level(p, h, F, S, i, j, k);
+  const int k0 = refl_melting_top(S, nk);
+  for (int k = k0 - 1; k >= 0; k--) refl_melting(h, F, S, k, k0);
+  for (int k = 0; k < nk; k++) refl_dbz(p, F, S, i, j, k);
 }
 
 }  // namespace morr
