@@ -123,8 +123,9 @@ int te_device_ptr(te_ctx *ctx, uint64_t word_off, void **out);
 int te_set_mode(te_ctx *ctx, int mode);
 
 /* Fused-mode plan of the active step (built on first use): segments are runs of exact
- * ops or fused phases.  kind: 0 = exact ops, 1 = acoustic substep (3 kernels),
- * 2 = periodic halo fills, 3 = advection of one variable (1 kernel).  te_run_segment
+ * ops or fused phases.  kind: 0 = exact ops, 1 = acoustic substep (2 kernels, 3 where the
+ * halos are filled: the last of a run), 2 = periodic halo fills, 3 = advection of one
+ * variable (1 kernel), 4 = mass fluxes and their divergence (1 or 2 kernels).  te_run_segment
  * plays one segment (part = -1) or one kernel of it (part >= 0), for profiling. */
 typedef struct te_segment {
   int kind;

@@ -11,6 +11,7 @@
 //       shared memory) and, after the last substep of a run of them, K3 (the four halo fills).
 //  * runs of periodic halo fills (bc_periodic_x then bc_periodic_y per field)
 //    -> one launch for up to four fields.
+//  * mass fluxes and their divergence (k_flux_div); every store kept.
 //
 // Contract: every field that is not step scratch (fpk, cA, cB are not written in fused
 // mode) ends bit-identical to the exact sequence; exact mode runs a phase fused only where
@@ -554,9 +555,82 @@ static void launch_halo(const HaloArgs& H, cudaStream_t s) {
   launch_kernel(k_halo_periodic, dim3(gr), dim3(b), 0, s, H);
 }
 
+// ------------------------------------------------------------ mass fluxes and their divergence
+
+// massflux_from_state then div_massflux (timestep.js:1904-1912), or divergence3d,
+// velocity_to_massflux then div_massflux (timestep.js:2093-2113).  One thread per point of the
+// field, numbered as in K1.  STATE: the mass fluxes are formed and stored, and the divergence
+// is taken of the neighbours' formed again, the same products (18 + 18.7 us as two launches at
+// 256x256x80, 35.6 us here).  Else: both divergences of the averaged velocities in one pass, the
+// scaled one of the products velocity_to_massflux then stores in place (16.8 + 18.7 us, 33 us
+// here; that launch follows).  Large grids gain little; on small ones it is two launches less
+// on the chain of each stage: fused 64x64x40 378 -> 335 us per step, 37x29x13 252 -> 242 us.
+struct FluxDivArgs {
+  Dims g;
+  const float *u, *v, *w;             // state (STATE) or averaged velocities
+  float *rru, *rrv, *rrw;             // mass fluxes (STATE)
+  const float *rho0, *rf0, *mh3, *mh, *hm;
+  float *div3d, *divx;
+};
+
+__device__ __forceinline__ float flux_div(const Dims& g, float u0, float u1, float v0, float v1, float w0, float w1, float mh,
+                                          float uh, float vh) {
+  return fmaf((w1 - w0) * g.rdz, mh, fmaf((u1 - u0) * g.rdx, uh, ((v1 - v0) * g.rdy) * vh));
+}
+
+template <bool STATE>
+__global__ void __launch_bounds__(256) k_flux_div(FluxDivArgs A, FastDiv dJ, FastDiv dK, unsigned total) {
+  const Dims& g = A.g;
+  const unsigned c = blockIdx.x * 256u + threadIdx.x;
+  if (c >= total) return;
+  const unsigned kk = fdiv(c, dK), r = c - kk * dK.d, jj = fdiv(r, dJ);
+  const int i = (int)(r - jj * dJ.d) - 3, j = (int)jj - 3, k = (int)kk;
+  if (i > g.nx + 3 || j > g.ny + 3) return;
+  const int sj = g.sJ, sk = g.sJ * g.sK;
+  const bool div = i <= g.nx + 2 && j <= g.ny + 2 && k < g.nz;
+  if (!STATE && !div) return;
+  const float w0 = A.w[c];
+  float u0 = 0.0f, v0 = 0.0f, u1 = 0.0f, v1 = 0.0f, w1 = 0.0f, rho = 0.0f;
+  if (k < g.nz) {
+    u0 = A.u[c];
+    v0 = A.v[c];
+    rho = A.rho0[k];
+  }
+  if (div) {
+    u1 = A.u[c + 1];
+    v1 = A.v[c + sj];
+    if (!STATE || k + 1 < g.nz) w1 = A.w[c + sk];
+  }
+  const float rw0 = (k == 0 || k == g.nz) ? 0.0f : A.rf0[k] * w0;
+  const float rw1 = k + 1 < g.nz ? A.rf0[k + 1] * w1 : 0.0f;
+  if (STATE) {
+    if (k < g.nz) {
+      A.rru[c] = rho * u0;
+      A.rrv[c] = rho * v0;
+    }
+    A.rrw[c] = rw0;
+  }
+  if (!div) return;
+  const float uh = hm_uh(g, A.hm, i), vh = hm_vh(g, A.hm, j);
+  if (!STATE && i >= 0 && j >= 0 && i < g.nx && j < g.ny) {
+    const float d = flux_div(g, u0, u1, v0, v1, w0, w1, A.mh3[k], uh, vh);
+    A.div3d[c] = fabsf(d) < 1e-30f ? 0.0f : d;
+  }
+  A.divx[c] = flux_div(g, rho * u0, rho * u1, rho * v0, rho * v1, rw0, rw1, A.mh[k], uh, vh);
+}
+
+static void launch_flux_div(const FluxDivArgs& A, cudaStream_t s) {
+  const Dims& g = A.g;
+  const unsigned total = (unsigned)g.sJ * (unsigned)g.sK * (unsigned)(g.nz + 1);
+  const dim3 gr((total + 255u) / 256u);
+  const FastDiv dJ = fast_div((unsigned)g.sJ), dK = fast_div((unsigned)g.sJ * (unsigned)g.sK);
+  if (A.rru) launch_kernel(k_flux_div<true>, gr, dim3(256), 0, s, A, dJ, dK, total);
+  else launch_kernel(k_flux_div<false>, gr, dim3(256), 0, s, A, dJ, dK, total);
+}
+
 // ------------------------------------------------------------ planner helpers
 
-enum SegKind { kExact = 0, kAcoustic = 1, kHalo = 2, kAdvect = 3 };
+enum SegKind { kExact = 0, kAcoustic = 1, kHalo = 2, kAdvect = 3, kFluxDiv = 4 };
 
 static bool is_name(const Op& o, const char* n) { return !o.copy && o.name == n; }
 
@@ -1114,10 +1188,81 @@ static bool match_substep(const std::vector<Op>& ops, size_t i, FusedSegment& s,
   return true;
 }
 
+// No field written is read or written twice, and none overlaps another.
+static bool separate_fields(const Plan& P, const std::vector<const float*>& wr, const std::vector<const float*>& rd) {
+  for (size_t a = 0; a < wr.size(); a++) {
+    if (!wr[a]) return false;
+    const Access x = P.access(wr[a], true);
+    for (size_t b = 0; b < wr.size() + rd.size(); b++) {
+      const float* f = b < wr.size() ? wr[b] : rd[b - wr.size()];
+      if (b == a) continue;
+      if (!f) return false;
+      const Access y = P.access(f, false);
+      if (x.lo < y.hi && y.lo < x.hi) return false;
+    }
+  }
+  return true;
+}
+
+static bool covers_field(const Op& o, int levels) {
+  const Dims& g = o.args.g;
+  return o.grid[0] >= g.nx + 7 && o.grid[1] >= g.ny + 7 && o.grid[2] >= levels;
+}
+
+static bool match_flux_div(const Plan& P, const std::vector<Op>& ops, size_t i, FusedSegment& s, FluxDivArgs& A) {
+  if (i + 2 > ops.size() || ops[i].copy) return false;
+  const bool state = is_name(ops[i], "massflux_from_state");
+  if (!state && !is_name(ops[i], "divergence3d")) return false;
+  const size_t n = state ? 2 : 3;
+  if (i + n > ops.size()) return false;
+  const Op &first = ops[i], &mf = ops[i + n - 2], &dv = ops[i + n - 1];
+  if (!is_name(mf, state ? "massflux_from_state" : "velocity_to_massflux") || !is_name(dv, "div_massflux")) return false;
+  const Dims& g = dv.args.g;
+  if (!same_dims(g, mf.args.g) || !same_dims(g, first.args.g)) return false;
+  if (!covers_field(mf, g.nz + 1) || !covers_field(dv, g.nz)) return false;
+  std::memset(&A, 0, sizeof A);
+  A.g = g;
+  A.mh = dv.args.p[4];
+  A.hm = dv.args.p[30];
+  A.divx = dv.args.p[5];
+  float* const* flux = state ? mf.args.p + 6 : mf.args.p + 3;
+  for (int q = 0; q < 3; q++)
+    if (dv.args.p[1 + q] != flux[q]) return false;
+  if (state) {
+    A.u = mf.args.p[1];
+    A.v = mf.args.p[2];
+    A.w = mf.args.p[3];
+    A.rru = flux[0];
+    A.rrv = flux[1];
+    A.rrw = flux[2];
+    A.rho0 = mf.args.p[4];
+    A.rf0 = mf.args.p[5];
+    if (!separate_fields(P, {A.rru, A.rrv, A.rrw, A.divx}, {A.u, A.v, A.w, A.rho0, A.rf0, A.mh, A.hm})) return false;
+  } else {
+    for (int q = 0; q < 3; q++)
+      if (first.args.p[1 + q] != flux[q]) return false;
+    if (first.grid[0] < g.nx || first.grid[1] < g.ny || first.grid[2] < g.nz || first.args.p[30] != A.hm) return false;
+    A.u = flux[0];
+    A.v = flux[1];
+    A.w = flux[2];
+    A.rho0 = mf.args.p[1];
+    A.rf0 = mf.args.p[2];
+    A.mh3 = first.args.p[4];
+    A.div3d = first.args.p[5];
+    if (!separate_fields(P, {A.div3d, A.divx}, {A.u, A.v, A.w, A.rho0, A.rf0, A.mh, A.mh3, A.hm})) return false;
+    if (!separate_fields(P, {A.u, A.v, A.w}, {A.rho0, A.rf0, A.mh, A.mh3, A.hm})) return false;
+  }
+  s.kind = kFluxDiv;
+  s.first = (int)i;
+  s.last = (int)(i + n - 1);
+  return true;
+}
+
 struct FusedData {
   std::vector<AcuArgs> acu;
   std::vector<HaloArgs> halo;
   std::vector<AdvArgs> adv;
+  std::vector<FluxDivArgs> flux;
 };
 
 // The words each kernel of a fused phase reads and writes (the phase's scratch fields that
@@ -1326,6 +1471,7 @@ void FusedStep::build(Plan& P, std::vector<Op>& ops, bool keep_scratch) {
   D.acu.clear();
   D.halo.clear();
   D.adv.clear();
+  D.flux.clear();
   size_t i = 0;
   auto exact_to = [&](size_t e) {
     if (!segs.empty() && segs.back().kind == kExact && segs.back().last + 1 == (int)i) segs.back().last = (int)e;
@@ -1351,6 +1497,14 @@ void FusedStep::build(Plan& P, std::vector<Op>& ops, bool keep_scratch) {
     if (match_advect(ops, i, P.M, s, V)) {
       s.aux[0] = (int)D.adv.size();
       D.adv.push_back(V);
+      segs.push_back(s);
+      i = s.last + 1;
+      continue;
+    }
+    FluxDivArgs X;
+    if (match_flux_div(P, ops, i, s, X)) {
+      s.aux[0] = (int)D.flux.size();
+      D.flux.push_back(X);
       segs.push_back(s);
       i = s.last + 1;
       continue;
@@ -1402,6 +1556,16 @@ void FusedStep::launch(Plan& P, std::vector<Op>& ops, StepDeps* deps) {
     if (s.kind == kExact) P.launch_exact(ops, s.first, s.last, false, deps);
     else if (s.kind == kHalo) run(halo_accesses(P, D.halo[s.aux[0]]), q, -1);
     else if (s.kind == kAdvect) run(adv_accesses(P, D.adv[s.aux[0]], s.aux[1]), q, -1);
+    else if (s.kind == kFluxDiv) {
+      const FluxDivArgs& A = D.flux[s.aux[0]];
+      std::vector<Access> acc;
+      for (const float* f : {A.u, A.v, A.w, A.rho0, A.rf0, A.mh3, A.mh, A.hm})
+        if (f) acc.push_back(P.access(f, false));
+      for (float* f : {A.rru, A.rrv, A.rrw, A.div3d, A.divx})
+        if (f) acc.push_back(P.access(f, true));
+      run(acc, q, 0);
+      if (!A.rru) run(P.accesses(ops[s.first + 1]), q, 1);
+    }
     else
       for (int part = 0; part < 2 + D.acu[s.aux[0]].fill; part++) run(acu_accesses(P, D.acu[s.aux[0]], part), q, part);
   }
@@ -1414,6 +1578,10 @@ void FusedStep::launch_segment(Plan& P, std::vector<Op>& ops, int seg, int part)
     P.launch_exact(ops, s.first, s.last, false);
   } else if (s.kind == kHalo) {
     launch_halo(D.halo[s.aux[0]], P.stream);
+  } else if (s.kind == kFluxDiv) {
+    const FluxDivArgs& A = D.flux[s.aux[0]];
+    if (part <= 0) launch_flux_div(A, P.stream);
+    if (!A.rru && part != 0) P.launch_exact(ops, s.first + 1, s.first + 1, false);  // velocity_to_massflux
   } else if (s.kind == kAdvect) {
     launch_adv(D.adv[s.aux[0]], s.aux[1], s.aux[2], P.stream);
   } else {
@@ -1438,6 +1606,7 @@ void FusedStep::launch_segment(Plan& P, std::vector<Op>& ops, int seg, int part)
 int FusedStep::kernels(int seg) const {
   const FusedSegment& s = segs.at(seg);
   if (s.kind == kExact) return 0;
+  if (s.kind == kFluxDiv) return static_cast<FusedData*>(data)->flux[s.aux[0]].rru ? 1 : 2;
   return s.kind == kAcoustic ? 2 + static_cast<FusedData*>(data)->acu[s.aux[0]].fill : 1;
 }
 
