@@ -120,6 +120,8 @@ void Plan::load_kernel_meta(const char* kjson, size_t klen) {
     const KernelSpec* t = kernel_table(&n);
     for (int i = 0; i < n; i++) {
       KMeta m;
+      // words of per-thread scratch, as kernels.json sizes them
+      m.scratch = !std::strcmp(t[i].name, "morr_column") ? 3712 : !std::strcmp(t[i].name, "morr_refl10cm") ? 1408 : 0;
       for (int q = 0; q < t[i].nparams; q++)
         m.params.push_back({t[i].params[q].index, t[i].params[q].kind != kPtr, t[i].params[q].write != 0});
       kmeta[t[i].name] = m;
