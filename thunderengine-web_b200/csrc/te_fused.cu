@@ -837,8 +837,149 @@ __global__ void __launch_bounds__(kAdvTX* kAdvTY, AdvMinBlocks<KIND>::value) k_a
     adv_tile<KIND, ST, false, OPEN>(A, fxs, fys);
 }
 
+// The 5th-order linear scalar advection (RK stages 1-2) of large grids.  k_adv_fused spends 376
+// instructions a cell there, two z faces, shared-memory faces and a barrier a level among
+// them.  Here a warp covers 31 cells of x (lane l computes x face l and takes face l + 1 from
+// its neighbour by shuffle) and kLinRows rows, and walks up the levels with the six-point z
+// stencil of each row in registers: 3.5 faces a cell instead of 4.2, no shared memory, no
+// barrier; every value of a level is requested before the first is used.  One B200,
+// per launch, th with the theta term / qv: 256x256x80 85 / 82 -> 71 / 66 us, 400x300x80 158 / 152
+// -> 111 / 104 us, 640x512x20 105 / 101 -> 80 / 75 us, 192x192x64 (2688 warps) 39 / 35 -> 37 /
+// 33 us; 128x128x64 (1280 warps) 18.6 -> 26 us, so from 16 warps an SM.  Measured beside it at
+// 256x256x80: 1 row a thread 77 / 72 us, 3 rows 78 / 69, 4 rows (spilling) 112 / 84; the
+// staggered and WENO kinds in this form no faster than k_adv_fused.
+constexpr int kLinRows = 2, kLinX = 31, kLinWarps = 4, kLinLevels = 16;
+
+__device__ __forceinline__ float lin_flux(float m, float v0, float v1, float v2, float v3, float v4, float v5) {
+  const bool up = m >= 0.0f;
+  return m * flx5(up ? v0 : v5, up ? v1 : v4, up ? v2 : v3, up ? v3 : v2, up ? v4 : v1);
+}
+
+template <bool OPEN>
+__global__ void __launch_bounds__(32 * kLinWarps, 6) k_adv_lin(AdvArgs A) {
+  constexpr int RY = kLinRows;
+  const Dims& g = A.as.g;
+  const int sj = g.sJ, sk = g.sJ * g.sK;
+  const int lane = threadIdx.x;
+  const int i = A.ilo + (int)blockIdx.x * kLinX + lane;
+  const int j0 = A.jlo + ((int)blockIdx.y * kLinWarps + (int)threadIdx.y) * RY;
+  if (j0 > A.jhi) return;  // whole warps; the warps of a block are independent
+  const int kb = A.klo + (int)blockIdx.z * kLinLevels, ke = min(A.khi, kb + kLinLevels - 1);
+  const bool cell = lane < kLinX && i <= A.ihi;
+  const int rmax = A.jhi - j0;  // the last row with cells, from j0
+  // lanes and rows past the last face repeat the last one's loads and store nothing
+  const int c00 = gidx(g, min(i, A.ihi + 1), j0, 0);
+  const float *a = A.as.p[2], *rru = A.fx.p[2], *rrv = A.fy.p[2], *rrw = A.fz.p[2], *divx = A.as.p[6], *hm = A.as.p[30];
+  const float mx = hm_uh(g, hm, min(i, A.ihi));
+  const bool thm = A.thterm != nullptr, rk = A.phi != nullptr, acc = A.accumulate != 0;
+  float q[RY][6], fzb[RY], my[RY];
+  int ro[RY];  // word offsets of the rows from j0
+#pragma unroll
+  for (int r = 0; r < RY; r++) {
+    ro[r] = min(r, rmax) * sj;
+    const int c = c00 + ro[r];
+    my[r] = hm_vh(g, hm, j0 + min(r, rmax));
+#pragma unroll
+    for (int t = 0; t < 6; t++) q[r][t] = __ldg(a + c + min(max(kb - 2 + t, 0), g.nz) * sk);
+    fzb[r] = cell ? face_lin_z_c(A.fz, g, c + kb * sk, kb) : 0.0f;
+    if (A.fzo && kb == A.klo && cell && r <= rmax) A.fzo[c + kb * sk] = fzb[r];  // the column's lowest face
+  }
+  for (int k = kb; k <= ke; k++) {
+    const int ck = c00 + k * sk;
+    float yv[RY + 6], mym[RY + 1], xs[RY][5], mxm[RY], mzm[RY], d0[RY], e0[RY], e1[RY], e2[RY], qn[RY];
+    const bool zin = k + 1 > 2 && k + 1 < g.nz - 2;  // the face above has the interior stencil
+#pragma unroll
+    for (int r = 0; r < RY; r++) {
+      const int c = ck + ro[r];
+      const float* ar = a + c;
+      xs[r][0] = __ldg(ar - 3);
+      xs[r][1] = __ldg(ar - 2);
+      xs[r][2] = __ldg(ar - 1);
+      xs[r][3] = __ldg(ar + 1);
+      xs[r][4] = __ldg(ar + 2);
+      mxm[r] = __ldg(rru + c);
+      if (zin) mzm[r] = __ldg(rrw + c + sk);
+      d0[r] = __ldg(divx + c);
+      if (acc) e0[r] = A.dest[c];
+      if (thm) {
+        e0[r] = __ldg(A.div3d + c);
+        e1[r] = __ldg(A.thterm + c);
+      }
+      if (rk) e2[r] = A.phiA[c];
+      qn[r] = __ldg(a + c00 + ro[r] + min(k + 4, g.nz) * sk);
+    }
+    // rows j0 - 3 .. j0 + RY + 2, the rows of cells from the z queues
+#pragma unroll
+    for (int t = 0; t < RY + 6; t++) {
+      const int r = t - 3;
+      if (r < 0 || r >= RY) yv[t] = __ldg(a + ck + min(r, rmax + 3) * sj);
+      else yv[t] = q[r < 0 ? 0 : (r < RY ? r : 0)][2];
+    }
+    if (rmax + 1 < RY) {  // the last group: rows past the cells, up to the last face's stencil
+#pragma unroll
+      for (int r = 1; r < RY; r++)
+        if (r > rmax) yv[r + 3] = __ldg(a + ck + min(r, rmax + 3) * sj);
+    }
+#pragma unroll
+    for (int r = 0; r <= RY; r++) mym[r] = __ldg(rrv + ck + min(r, rmax + 1) * sj);
+    const float mz = __ldg(A.as.p[9] + k), rho = __ldg(A.as.p[7] + k);
+    float fy[RY + 1], fx[RY], fzt[RY];
+#pragma unroll
+    for (int r = 0; r <= RY; r++) fy[r] = lin_flux(mym[r], yv[r], yv[r + 1], yv[r + 2], yv[r + 3], yv[r + 4], yv[r + 5]);
+#pragma unroll
+    for (int r = 0; r < RY; r++) {
+      fx[r] = lin_flux(mxm[r], xs[r][0], xs[r][1], xs[r][2], q[r][2], xs[r][3], xs[r][4]);
+      if (zin) fzt[r] = lin_flux(mzm[r], q[r][0], q[r][1], q[r][2], q[r][3], q[r][4], q[r][5]);
+      else fzt[r] = cell ? face_lin_z_c(A.fz, g, ck + ro[r] + sk, k + 1) : 0.0f;
+    }
+    if (A.fxo) {  // each face by the tile that has its upper cell, the last one by the last tile
+#pragma unroll
+      for (int r = 0; r <= RY; r++) {
+        const int c = ck + r * sj;
+        if (r < RY && r <= rmax) {
+          if (cell || i == A.ihi + 1) A.fxo[c] = fx[r < RY ? r : 0];
+          if (cell) A.fzo[c + sk] = fzt[r < RY ? r : 0];
+        }
+        if (cell && r <= rmax + 1 && (r < RY || r == rmax + 1)) A.fyo[c] = fy[r];
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < RY; r++) {
+      const float dFx = __shfl_down_sync(0xffffffffu, fx[r], 1) - fx[r], dFy = fy[r + 1] - fy[r];
+      if (cell && r <= rmax) {
+        const int c = ck + r * sj;
+        float dv = d0[r], gx = dFx, gy = dFy;
+        if (OPEN) assemble_open<1>(A.as, i, j0 + r, k, c, gx, gy, dv);
+        const float divF = fmaf((fzt[r] - fzb[r]) * g.rdz, mz, fmaf(gx * g.rdx, mx, (gy * g.rdy) * my[r]));
+        float tn = dcr(fmaf(q[r][2], dv, -divF), rho);
+        if (acc) {
+          A.dest[c] = e0[r] + tn;
+        } else {
+          if (thm) tn = fmaf(-e0[r], e1[r], tn);        // apply_thterm.wgsl
+          if (A.write_dest) A.dest[c] = tn;
+          if (rk) A.phi[c] = fmaf(A.dttmp, tn, e2[r]);  // rk_update.wgsl
+        }
+      }
+      fzb[r] = fzt[r];
+#pragma unroll
+      for (int t = 0; t < 5; t++) q[r][t] = q[r][t + 1];
+      q[r][5] = qn[r];
+    }
+  }
+}
+
 template <int KIND, int ST>
 static void launch_adv_t(const AdvArgs& A, cudaStream_t s) {
+  if (KIND == kLin) {
+    const int strips = (A.ihi - A.ilo + kLinX) / kLinX, rows = (A.jhi - A.jlo + kLinRows) / kLinRows;
+    const int walks = (A.khi - A.klo + kLinLevels) / kLinLevels;
+    if ((long)strips * rows * walks >= 148 * 16) {  // below, walks of 16 levels leave the chip idle
+      const dim3 gr(strips, (rows + kLinWarps - 1) / kLinWarps, walks), bl(32, kLinWarps);
+      if (A.open) launch_kernel(k_adv_lin<true>, gr, bl, 0, s, A);
+      else launch_kernel(k_adv_lin<false>, gr, bl, 0, s, A);
+      return;
+    }
+  }
   const dim3 b(kAdvTX, kAdvTY, 1);
   constexpr int kz = AdvKZ<KIND>::value;
   const dim3 gr((A.ihi - A.ilo + kAdvTX) / kAdvTX, (A.jhi - A.jlo + kAdvTY) / kAdvTY, (A.khi - A.klo + kz) / kz);
