@@ -775,10 +775,15 @@ void launch_step(Plan& P, AdjointState& S, AdjointState::StepGraph& G, uint64_t 
     cudaGraphExec_t exec = nullptr;
     const cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
     cudaGraphDestroy(graph);
-    ACU(e);
-    G.chain = G.exec;
-    G.exec = exec;
-    G.concurrent = upgrade;
+    if (e != cudaSuccess && upgrade) {  // the chain stays
+      cudaGetLastError();
+      G.concurrent = true;
+    } else {
+      ACU(e);
+      G.chain = G.exec;
+      G.exec = exec;
+      G.concurrent = upgrade;
+    }
   }
   launch_kernel(adj::k_set_word, dim3(1), dim3(1), 0, P.stream, S.log_at, log);
   ACU(cudaGraphLaunch(G.exec, P.stream));

@@ -3,6 +3,7 @@
 // for repeated steps, fused step phases in TE_MODE_FUSED (te_fused.cu).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -149,14 +150,12 @@ std::map<int, uint64_t> Plan::layout_bytes(const JValue& cmds) {
 
 uint64_t Plan::region_len(uint64_t off) const {
   // regionLen (replay.js:168-178): arena field or rest of the buffer
-  for (int b = (int)buffers.size() - 1; b >= 0; b--) {
-    if (off >= base[b]) {
-      uint64_t end = base[b] + buffers[b].length / 4;
-      if (buffers[b].arena) return std::min<uint64_t>(field_stride / 4, end - off);
-      return end - off;
-    }
-  }
-  return 0;
+  const size_t n = std::upper_bound(base.begin(), base.end(), off) - base.begin();
+  if (!n) return 0;
+  const BufInfo& b = buffers[n - 1];  // the last buffer that starts at or before off
+  const uint64_t end = base[n - 1] + b.length / 4;
+  if (b.arena) return std::min<uint64_t>(field_stride / 4, end - off);
+  return end - off;
 }
 
 std::vector<Op> Plan::build_ops(const JValue& cmds, const std::map<int, uint64_t>& offs, bool hashes) {
@@ -887,10 +886,15 @@ void Plan::launch_step_graph() {
     cudaGraphExec_t exec = nullptr;
     const cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
     cudaGraphDestroy(graph);
-    CU(e);
-    graph_chain = graph_exec;
-    graph_exec = exec;
-    graph_concurrent = upgrade;
+    if (e != cudaSuccess && upgrade) {  // the chain stays
+      cudaGetLastError();
+      graph_concurrent = true;
+    } else {
+      CU(e);
+      graph_chain = graph_exec;
+      graph_exec = exec;
+      graph_concurrent = upgrade;
+    }
   }
   CU(cudaGraphLaunch(graph_exec, stream));
   if (graph_runs < kChainRuns) graph_runs++;
