@@ -8,7 +8,7 @@ from tests.test_morr import host_kernels, morr_case, refl_case
 
 
 # columns of the recording's 40 levels with seeded condensate; 33 x 5 columns (a ragged block) of
-# fewer levels than warps, and of one level
+# fewer levels than warps, of one level, and of a level count that is no multiple of the warps
 @pytest.mark.gpu
 @pytest.mark.parametrize('variant,seed,nx,ny,nz', [('random', 1, 50, 9, 40), ('supersaturated', 3, 50, 9, 40),
                                                    ('random', 5, 33, 5, 7), ('supersaturated', 6, 33, 5, 1),

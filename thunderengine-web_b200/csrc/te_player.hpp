@@ -82,7 +82,7 @@ struct Plan {
   cudaGraphExec_t graph_exec = nullptr;
   cudaGraphExec_t graph_chain = nullptr;  // the chain a concurrent graph_exec replaced, which may still run
   int graph_runs = 0;             // steps launched since the step, mode or parameters last changed
-  bool graph_concurrent = false;  // graph_exec holds the data's orders only, not the whole chain
+  bool graph_concurrent = false;  // the concurrent form was made (or could not be: the chain stays)
   FusedStep fused;        // the active step in fused mode
   FusedStep exact_fused;  // in exact mode: the phases whose every store the step repeats, fused
   bool fused_dirty = true, exact_dirty = true;
