@@ -1331,17 +1331,16 @@ static bool match_substep(const std::vector<Op>& ops, size_t i, FusedSegment& s,
 
 // No field written is read or written twice, and none overlaps another.
 static bool separate_fields(const Plan& P, const std::vector<const float*>& wr, const std::vector<const float*>& rd) {
-  for (size_t a = 0; a < wr.size(); a++) {
-    if (!wr[a]) return false;
-    const Access x = P.access(wr[a], true);
-    for (size_t b = 0; b < wr.size() + rd.size(); b++) {
-      const float* f = b < wr.size() ? wr[b] : rd[b - wr.size()];
-      if (b == a) continue;
+  std::vector<Access> all;
+  all.reserve(wr.size() + rd.size());
+  for (const auto* fields : {&wr, &rd})
+    for (const float* f : *fields) {
       if (!f) return false;
-      const Access y = P.access(f, false);
-      if (x.lo < y.hi && y.lo < x.hi) return false;
+      all.push_back(P.access(f, false));
     }
-  }
+  for (size_t a = 0; a < wr.size(); a++)
+    for (size_t b = a + 1; b < all.size(); b++)
+      if (all[a].lo < all[b].hi && all[b].lo < all[a].hi) return false;
   return true;
 }
 
@@ -1458,7 +1457,7 @@ static std::vector<Access> acu_accesses(const Plan& P, const AcuArgs& A, int par
   return acc;
 }
 
-// Runs of consecutive substeps on one set of fields skip the halo fills between them (K1).
+// Runs of consecutive substeps on one set of fields (plain_bindings) skip the halo fills between them (K1).
 // u and v alternate between their fields and the two workspace fields; the first substep
 // may stay in place (it does not wrap), so that an even number of changes ends in the fields.
 static void chain_substeps(const Plan& P, std::vector<FusedSegment>& segs, std::vector<AcuArgs>& acu) {
@@ -1520,36 +1519,30 @@ static StoreKey store_key(const Op& o, const float* out) {
                   g.sJ, g.sK, o.name == "adv_assemble" ? o.args.iv[1] : 0};
 }
 
-// The regions the ops of a phase bind are equal or disjoint, and nothing a phase's fused
-// kernels write or skip is read by them in another role.
-static bool plain_bindings(const Plan& P, const std::vector<Op>& ops, const std::vector<std::vector<Access>>& acc,
-                           const FusedSegment& s, const FusedData& D) {
-  std::vector<Access> all;
-  for (int q = s.first; q <= s.last; q++) all.insert(all.end(), acc[q].begin(), acc[q].end());
-  std::sort(all.begin(), all.end(), [](const Access& a, const Access& b) { return a.lo < b.lo; });
-  for (size_t q = 1; q < all.size(); q++)
-    if (all[q].lo != all[q - 1].lo && all[q].lo < all[q - 1].hi) return false;
+// What a phase writes, in its ops or its fused kernels, is a field of its own: no other binding
+// of the phase names or overlaps it.  Phases of other bindings run per dispatch, in either mode:
+// a run of substeps moves u and v to the workspace and leaves halos unfilled (chain_substeps), and
+// a fused kernel's order of loads and stores is not that of the ops it stands for.
+static bool plain_bindings(const Plan& P, const std::vector<Op>& ops, const FusedSegment& s, const FusedData& D) {
   std::vector<const float*> wr, rd;
   if (s.kind == kAcoustic) {
     const AcuArgs& A = D.acu[s.aux[0]];
     const Op &fp = ops[s.first + 1], &ws = ops[s.first + 2];
     wr = {A.ppd, A.u, A.v, A.w, A.rru, A.rrv, A.rrw, A.pp3d, A.ppx, fp.args.p[11], ws.args.p[10], ws.args.p[11]};
     rd = {A.thv, A.uten, A.vten, A.hm, A.piadv, A.ppten, A.ppterm, A.pk1, A.pk2, A.qk, A.mm, A.wten};
-    if (A.ppd != A.ppdw) return false;
   } else if (s.kind == kAdvect) {
     const AdvArgs& A = D.adv[s.aux[0]];
     const KArgs& as = ops[s.first + 3].args;
     wr = {A.dest, as.p[3], as.p[4], as.p[5]};
     if (A.phi) wr.push_back(A.phi);
     for (const Access& a : adv_reads(P, A, s.aux[1])) rd.push_back(reinterpret_cast<const float*>(a.lo));
+  } else if (s.kind == kHalo) {
+    const HaloArgs& H = D.halo[s.aux[0]];
+    wr.assign(H.f, H.f + H.nf);
+  } else {
+    return true;  // kFluxDiv: match_flux_div
   }
-  std::sort(wr.begin(), wr.end());
-  for (size_t q = 0; q < wr.size(); q++) {
-    if (!wr[q] || (q && wr[q] == wr[q - 1])) return false;
-    for (const float* r : rd)
-      if (r == wr[q]) return false;
-  }
-  return true;
+  return separate_fields(P, wr, rd);
 }
 
 // keep_scratch (exact mode): a phase stays fused when every store it skips is made again later in the step,
@@ -1572,8 +1565,8 @@ static void keep_final_stores(const Plan& P, const std::vector<Op>& ops, std::ve
   };
   for (size_t n = segs.size(); n-- > 0;) {
     FusedSegment& s = segs[n];
-    bool keep = s.kind == kExact || plain_bindings(P, ops, acc, s, D);
-    if (keep && s.kind != kExact) {
+    bool keep = true;
+    if (s.kind != kExact) {
       for (const Skipped& k : skipped_stores(ops, s, D)) {
         const StoreKey key = store_key(ops[k.op], k.out);
         if (!later.count(key)) keep = false;
@@ -1596,13 +1589,6 @@ static void keep_final_stores(const Plan& P, const std::vector<Op>& ops, std::ve
       for (int q = 0; q < 3; q++) add(ops[s.first + q]);
     }
   }
-  // adjacent exact runs in one
-  std::vector<FusedSegment> out;
-  for (const FusedSegment& s : segs) {
-    if (s.kind == kExact && !out.empty() && out.back().kind == kExact) out.back().last = s.last;
-    else out.push_back(s);
-  }
-  segs.swap(out);
 }
 
 void FusedStep::build(Plan& P, std::vector<Op>& ops, bool keep_scratch) {
@@ -1678,7 +1664,16 @@ void FusedStep::build(Plan& P, std::vector<Op>& ops, bool keep_scratch) {
     exact_to(i);
     i++;
   }
+  for (FusedSegment& s : segs)
+    if (s.kind != kExact && !plain_bindings(P, ops, s, D)) s.kind = kExact;
   if (keep_scratch) keep_final_stores(P, ops, segs, D);
+  // adjacent exact runs in one
+  std::vector<FusedSegment> out;
+  for (const FusedSegment& s : segs) {
+    if (s.kind == kExact && !out.empty() && out.back().kind == kExact) out.back().last = s.last;
+    else out.push_back(s);
+  }
+  segs.swap(out);
   chain_substeps(P, segs, D.acu);
 }
 
