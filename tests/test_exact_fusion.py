@@ -1,5 +1,8 @@
 """Exact mode runs a phase fused where the step stores the phase's scratch again later.  Every
 memory word after a step must be the one the ops in tape order leave."""
+import base64
+import struct
+
 import numpy as np
 import pytest
 
@@ -108,4 +111,62 @@ def test_aliased_substeps(pipe, index, field, words, mode):
     run = _run()
     tape = run.tape(1)
     _bind(tape, pipe, index, run.fields[field] + 4 * words)
+    _same_words(run, tape, run.initial_buffers(), mode)
+
+
+# qv's x faces of stage 1 but the last: its assembly reads that one as th's dispatch left it.
+@pytest.mark.gpu
+@pytest.mark.parametrize('mode', [0, 1])
+def test_a_flux_dispatch_of_a_part_of_the_faces(mode):
+    run = _run()
+    tape = run.tape(1)
+    at = [q for q, c in enumerate(tape['steps'][0]) if c['op'] == 'pipe' and c['name'] == 'adv_flux_x'][1]
+    next(c for c in tape['steps'][0][at:] if c['op'] == 'dispatch')['grid'] = [run.grid.nx, run.grid.ny, run.grid.nz]
+    _same_words(run, tape, run.initial_buffers(), mode)
+
+
+def _probe(tape, run):
+    """A further buffer of one field, outside the arena."""
+    tape['buffers'].append(dict(id=len(tape['buffers']), label='probe', length=run.grid.count * 4))
+    return tape['buffers'][-1]['id']
+
+
+def _adv_u(tape, run, stage, opened, after):
+    """u's assembly of RK stage `stage` stores its tendency in `tend` instead of adding it to uten,
+    with open x edges (whose faces keep what tend held) or closed ones; `after` follows it."""
+    now, seen, mine, out = None, -1, False, []
+    for c in tape['steps'][0]:
+        if c['op'] == 'pipe':
+            now, mine = c['name'], False
+        if now == 'adv_assemble' and c['op'] == 'bytes':
+            if c['index'] == 1:
+                u = struct.unpack('<i', base64.b64decode(c['data'])[:4])[0] == 2
+                seen += u
+                mine = u and seen == stage
+            elif mine and c['index'] == 12:
+                c['data'] = base64.b64encode(struct.pack('<i', 0)).decode()
+            elif mine and c['index'] == 17:
+                c['data'] = base64.b64encode(struct.pack('<ii', int(opened), 0)).decode()
+        if mine and c['op'] in ('buf', 'bufoff') and c['index'] == 11:
+            c['offset'] = run.fields['tend']
+        out.append(c)
+        if mine and c['op'] == 'dispatch':
+            out += after
+            mine = False
+    tape['steps'][0] = out
+    assert seen >= stage
+    _bind(tape, 'adv_assemble', 19, run.fields['qzero'])   # a field it does not use; by default tend too
+
+
+# An assembly of u on open edges leaves the tendency's edge faces alone, so a copy after it
+# reads there what th's assembly stored before it.
+@pytest.mark.gpu
+@pytest.mark.parametrize('mode', [0, 1])
+def test_open_edge_faces_of_a_shared_tendency(mode):
+    run = _run()
+    tape = run.tape(1)
+    _adv_u(tape, run, 1, True, [dict(op='copy', src=run.rec.ids['arena'], srcOffset=run.fields['tend'],
+                                     dst=_probe(tape, run), dstOffset=0, size=run.grid.count * 4)])
+    for pipe, index, only in (('adv_assemble', 11, 4), ('rk_update', 3, 1)):   # qv's tendency of stage 1 elsewhere
+        _bind(tape, pipe, index, run.fields['cA'], only)
     _same_words(run, tape, run.initial_buffers(), mode)

@@ -1018,8 +1018,9 @@ static const FluxNames kFluxSets[] = {
 };
 
 // Face indices a flux dispatch writes: its dispatch grid mapped to indices (the staggered
-// horizontal kernels start at -1), cut by the kernel's own range check (te_kernels.cu).
-static FaceRange flux_range(int kind, int dir, const Op& o) {
+// horizontal kernels start at -1), cut by the kernel's own range check (te_kernels.cu).  *whole:
+// the grid reaches the end of that range, so every such dispatch writes the same words.
+static FaceRange flux_range(int kind, int dir, const Op& o, bool* whole = nullptr) {
   const Dims& g = o.args.g;
   const bool centred = kind == kLin || kind == kWeno;
   const int off = !centred && dir != 2 ? -1 : 0;
@@ -1038,6 +1039,7 @@ static FaceRange flux_range(int kind, int dir, const Op& o) {
     r.ilo = std::max(r.ilo, 0);
     r.jlo = std::max(r.jlo, 0);
   }
+  if (whole) *whole = r.ihi >= gi && r.jhi >= gj && r.khi >= gk;
   r.ihi = std::min(r.ihi, gi);
   r.jhi = std::min(r.jhi, gj);
   r.khi = std::min(r.khi, gk);
@@ -1055,29 +1057,38 @@ static bool references(const Op& o, const float* f) {
   return false;
 }
 
+// adv_assemble leaves the boundary faces of u (v) on open x (y) edges alone (te_kernels.cu).
+static bool leaves_edges(const Op& assemble) {
+  const int st = std::abs(assemble.args.iv[1]);
+  return (st == 2 && assemble.args.iv[17] != 0) || (st == 3 && assemble.args.iv2[17] != 0);
+}
+
 // Does op o overwrite f everywhere it matters without reading it first?  Only the
 // flux kernels (their output binding) and adv_assemble without accumulation (its
-// tendency) are known to; any other kernel that names f counts as a reader.
+// tendency), over their whole range, are known to; any other kernel that names f counts as
+// a reader.
 static bool writes_first(const Op& o, const float* f) {
   const std::string& n = o.name;
+  int out = -1;
+  bool whole = false;
   for (auto& fs : kFluxSets) {
-    const bool h = n == fs.x || n == fs.y, z = n == fs.z;
-    if (!h && !z) continue;
-    const int out = h ? fs.out_h : fs.out_z;
-    for (int q = 0; q < o.spec->nparams; q++) {
-      const ParamSpec& ps = o.spec->params[q];
-      if (ps.kind == kPtr && ps.index != out && o.args.p[ps.index] == f) return false;
-    }
-    return o.args.p[out] == f;
+    const int dir = n == fs.x ? 0 : n == fs.y ? 1 : n == fs.z ? 2 : -1;
+    if (dir < 0) continue;
+    out = dir == 2 ? fs.out_z : fs.out_h;
+    flux_range(fs.kind, dir, o, &whole);
   }
   if (n == "adv_assemble" && o.args.iv[12] == 0) {
-    for (int q = 0; q < o.spec->nparams; q++) {
-      const ParamSpec& ps = o.spec->params[q];
-      if (ps.kind == kPtr && ps.index != 11 && o.args.p[ps.index] == f) return false;
-    }
-    return o.args.p[11] == f;
+    const Dims& g = o.args.g;
+    const int st = std::abs(o.args.iv[1]);
+    out = 11;
+    whole = !leaves_edges(o) && o.grid[0] >= g.nx + (st == 2) && o.grid[1] >= g.ny + (st == 3) && o.grid[2] >= g.nz;
   }
-  return false;
+  if (out < 0 || !whole) return false;
+  for (int q = 0; q < o.spec->nparams; q++) {
+    const ParamSpec& ps = o.spec->params[q];
+    if (ps.kind == kPtr && ps.index != out && o.args.p[ps.index] == f) return false;
+  }
+  return o.args.p[out] == f;
 }
 
 // The values ops [first, last] leave in field f are never read afterwards: scanning the
