@@ -1,6 +1,7 @@
 """Exact mode runs a phase fused where the step stores the phase's scratch again later.  Every
 memory word after a step must be the one the ops in tape order leave."""
 import base64
+import copy
 import struct
 
 import numpy as np
@@ -114,6 +115,18 @@ def test_aliased_substeps(pipe, index, field, words, mode):
     _same_words(run, tape, run.initial_buffers(), mode)
 
 
+# One substep whose column solve reads the coefficients the substep before it left, and stores its
+# own there or elsewhere.
+@pytest.mark.gpu
+@pytest.mark.parametrize('binds', [((7, 'cA'),), ((5, 'cB'),), ((7, 'cA'), (10, 'fx'))])
+def test_a_later_op_that_reads_skipped_scratch(binds):
+    run = _run()
+    tape = run.tape(1)
+    for index, field in binds:
+        _bind(tape, 'acoustic_w_solve', index, run.fields[field], only=4)
+    _same_words(run, tape, run.initial_buffers(), 0)
+
+
 # qv's x faces of stage 1 but the last: its assembly reads that one as th's dispatch left it.
 @pytest.mark.gpu
 @pytest.mark.parametrize('mode', [0, 1])
@@ -170,3 +183,28 @@ def test_open_edge_faces_of_a_shared_tendency(mode):
     for pipe, index, only in (('adv_assemble', 11, 4), ('rk_update', 3, 1)):   # qv's tendency of stage 1 elsewhere
         _bind(tape, pipe, index, run.fields['cA'], only)
     _same_words(run, tape, run.initial_buffers(), mode)
+
+
+# Closed edges in stage 1, open ones in stage 2: the second assembly does not store the faces
+# that the first one did.
+@pytest.mark.gpu
+def test_a_store_on_closed_edges_is_not_repeated_on_open_ones():
+    run = _run()
+    tape = run.tape(1)
+    probe = _probe(tape, run)
+    cmds = tape['steps'][0]
+    first = next(q for q, c in enumerate(cmds) if c['op'] == 'pipe' and c['name'] == 'rk_update')
+    rk = copy.deepcopy(cmds[first:first + 1 + next(q for q, c in enumerate(cmds[first:]) if c['op'] == 'dispatch')])
+    for c in rk:   # rk_update of u's tendency into the probe
+        if c['op'] == 'bytes' and c['index'] == 1:
+            c['data'] = base64.b64encode(struct.pack('<i', 2)).decode()
+        elif c['op'] == 'buf' and c['index'] in (2, 3):
+            c['offset'] = run.fields[{2: 'u_a', 3: 'tend'}[c['index']]]
+        elif c['op'] == 'buf' and c['index'] == 4:
+            c['buf'], c['offset'] = probe, 0
+        elif c['op'] == 'dispatch':
+            c['grid'] = [run.grid.nx + 1, run.grid.ny, run.grid.nz]
+    assert [c['index'] for c in rk if c['op'] == 'buf'] == [30, 2, 3, 4]
+    for stage, opened in ((0, False), (1, True)):
+        _adv_u(tape, run, stage, opened, copy.deepcopy(rk))
+    _same_words(run, tape, run.initial_buffers(), 0)

@@ -20,9 +20,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <array>
 #include <cstring>
-#include <set>
 #include <stdexcept>
 #include <string>
 
@@ -1521,13 +1519,42 @@ static std::vector<Skipped> skipped_stores(const std::vector<Op>& ops, const Fus
   return v;
 }
 
-// Two dispatches with equal keys write the same words: same kernel, output field, dispatch
-// grid, dimensions and (adv_assemble) stagger.
-typedef std::array<long long, 11> StoreKey;
-static StoreKey store_key(const Op& o, const float* out) {
+// Op o writes the words that op w writes to its output `out`: same kernel, output binding, dispatch
+// grid, dimensions and (adv_assemble) stagger and edges.
+static bool same_store(const Op& o, const Op& w, const float* out) {
+  if (o.spec != w.spec || !same_dims(o.args.g, w.args.g)) return false;
+  for (int d = 0; d < 3; d++)
+    if (o.grid[d] != w.grid[d]) return false;
+  if (w.name == "adv_assemble" && (o.args.iv[1] != w.args.iv[1] || leaves_edges(o) != leaves_edges(w))) return false;
+  for (int q = 0; q < w.spec->nparams; q++) {
+    const ParamSpec& ps = w.spec->params[q];
+    if (ps.kind == kPtr && ps.write && w.args.p[ps.index] == out && o.args.p[ps.index] != out) return false;
+  }
+  return true;
+}
+
+// The faces a flux dispatch writes into `out`.
+static bool flux_store(const Op& o, const float* out, FaceRange& r) {
+  for (auto& fs : kFluxSets) {
+    const int dir = o.name == fs.x ? 0 : o.name == fs.y ? 1 : o.name == fs.z ? 2 : -1;
+    if (dir < 0) continue;
+    r = flux_range(fs.kind, dir, o);
+    return o.args.p[dir == 2 ? fs.out_z : fs.out_h] == out;
+  }
+  return false;
+}
+
+// The faces of `out`, one of its three flux fields, that adv_assemble reads.
+static bool faces_read(const Op& o, const float* out, FaceRange& r) {
+  if (o.name != "adv_assemble") return false;
   const Dims& g = o.args.g;
-  return StoreKey{(long long)(uintptr_t)o.spec, (long long)(uintptr_t)out, o.grid[0], o.grid[1], o.grid[2], g.nx, g.ny, g.nz,
-                  g.sJ, g.sK, o.name == "adv_assemble" ? o.args.iv[1] : 0};
+  const int st = std::abs(o.args.iv[1]);
+  r = FaceRange{0, st == 2 ? g.nx : g.nx - 1, 0, st == 3 ? g.ny : g.ny - 1, st == 4 ? 1 : 0, g.nz - 1};
+  const int dir = out == o.args.p[3] ? 0 : out == o.args.p[4] ? 1 : out == o.args.p[5] ? 2 : -1;
+  if (dir == 0) (st == 2 ? r.ilo : r.ihi) += st == 2 ? -1 : 1;
+  if (dir == 1) (st == 3 ? r.jlo : r.jhi) += st == 3 ? -1 : 1;
+  if (dir == 2) (st == 4 ? r.klo : r.khi) += st == 4 ? -1 : 1;
+  return dir >= 0;
 }
 
 // What a phase writes, in its ops or its fused kernels, is a field of its own: no other binding
@@ -1556,49 +1583,48 @@ static bool plain_bindings(const Plan& P, const std::vector<Op>& ops, const Fuse
   return separate_fields(P, wr, rd);
 }
 
-// keep_scratch (exact mode): a phase stays fused when every store it skips is made again later in the step,
-// by a dispatch that writes the same words, before anything else touches the field.  The
-// last dispatch of each kind is then one that runs (or a fused phase that stores its
-// fluxes), so every word ends with the value of its last writer.  Of a moist step the last
-// substep and the last variable of each flux kind run per dispatch (333 launches -> 157).
+// keep_scratch (exact mode): a phase stays fused when every store it skips is made again later in
+// the step, by a dispatch that writes (at least) the same words without reading the field, and
+// nothing reads them before that.  Flux dispatches in between may write a part of the field and
+// assemblies read back what those wrote.  The later dispatch runs, or is itself skipped for one
+// that is later still, so every word ends with the value of its last writer.  Of a moist step the
+// last substep and the last variable of each flux kind run per dispatch (333 launches -> 124).
 // One B200, per step: exact 128x128x64 1.58 -> 1.26 ms, exact 12x10x8 280 -> 197 us; the
 // per-dispatch form spent the difference on launches and on writing and re-reading fluxes.
 static void keep_final_stores(const Plan& P, const std::vector<Op>& ops, std::vector<FusedSegment>& segs, const FusedData& D) {
   std::vector<std::vector<Access>> acc;
   for (const Op& o : ops) acc.push_back(P.accesses(o));
-  std::set<StoreKey> later;  // keys of the stores that segments after this one make
-  auto add = [&](const Op& o) {
-    if (o.copy || !o.spec) return;
-    for (int q = 0; q < o.spec->nparams; q++) {
-      const ParamSpec& ps = o.spec->params[q];
-      if (ps.kind == kPtr && ps.write && o.args.p[ps.index]) later.insert(store_key(o, o.args.p[ps.index]));
+  auto stored_again = [&](const Skipped& k, int last) {
+    const Op& w = ops[k.op];
+    const Access f = P.access(k.out, true);
+    FaceRange skipped, r, own{0, -1, 0, -1, 0, -1};  // own: faces written since
+    const bool flux = flux_store(w, k.out, skipped);
+    auto within = [](const FaceRange& a, const FaceRange& b) { return covers(b, a.ilo, a.ihi, a.jlo, a.jhi, a.klo, a.khi); };
+    for (size_t q = (size_t)last + 1; q < ops.size(); q++) {
+      int touches = 0;
+      for (const Access& a : acc[q]) touches += a.lo < f.hi && f.lo < a.hi;
+      if (!touches) continue;
+      const Op& o = ops[q];
+      if (o.copy || !o.spec || touches > 1 || !same_dims(o.args.g, w.args.g)) return false;
+      // its one binding on the field is the output (adv_assemble's accumulation reads it)
+      if (same_store(o, w, k.out)) return !(o.name == "adv_assemble" && o.args.iv[12] != 0);
+      if (flux && flux_store(o, k.out, r)) {
+        if (within(skipped, r)) return true;
+        own = r;
+      } else if (!(flux && faces_read(o, k.out, r) && within(r, own))) {
+        return false;
+      }
     }
+    return false;
   };
   for (size_t n = segs.size(); n-- > 0;) {
     FusedSegment& s = segs[n];
-    bool keep = true;
-    if (s.kind != kExact) {
-      for (const Skipped& k : skipped_stores(ops, s, D)) {
-        const StoreKey key = store_key(ops[k.op], k.out);
-        if (!later.count(key)) keep = false;
-        const Access f = P.access(k.out, true);
-        for (size_t q = (size_t)s.last + 1; keep && q < ops.size(); q++) {
-          bool touched = false;
-          for (const Access& a : acc[q]) touched |= a.lo < f.hi && f.lo < a.hi;
-          if (!touched) continue;
-          // the first op that touches the field writes it without reading it
-          keep = !ops[q].copy && (store_key(ops[q], k.out) == key || writes_first(ops[q], k.out));
-          break;
-        }
-        if (!keep) break;
+    if (s.kind == kExact) continue;
+    for (const Skipped& k : skipped_stores(ops, s, D))
+      if (!stored_again(k, s.last)) {
+        s.kind = kExact;
+        break;
       }
-    }
-    if (!keep) s.kind = kExact;
-    if (s.kind == kExact) {
-      for (int q = s.first; q <= s.last; q++) add(ops[q]);
-    } else if (s.kind == kAdvect && D.adv[s.aux[0]].fxo) {
-      for (int q = 0; q < 3; q++) add(ops[s.first + q]);
-    }
   }
 }
 
