@@ -126,7 +126,9 @@ int te_set_mode(te_ctx *ctx, int mode);
  * ops or fused phases.  kind: 0 = exact ops, 1 = acoustic substep (2 kernels, 3 where the
  * halos are filled: the last of a run), 2 = periodic halo fills, 3 = advection of one
  * variable (1 kernel), 4 = mass fluxes and their divergence (1 or 2 kernels).  te_run_segment
- * plays one segment (part = -1) or one kernel of it (part >= 0), for profiling. */
+ * plays one segment (part = -1), which leaves every field but the step's scratch as its ops do, or one
+ * kernel of it as the step runs it (part >= 0), for profiling: within a run of substeps
+ * u and v then pass through the player's workspace. */
 typedef struct te_segment {
   int kind;
   int first_op, last_op;

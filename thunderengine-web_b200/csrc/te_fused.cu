@@ -1714,6 +1714,23 @@ void FusedStep::build(Plan& P, std::vector<Op>& ops, bool keep_scratch) {
   chain_substeps(P, segs, D.acu);
 }
 
+// Kernel `part` of a substep, or (part < 0) all of them.
+static void launch_substep(const AcuArgs& A, int part, cudaStream_t s) {
+  if (part < 0 || part == 0) launch_acu_uv(A, s);
+  if (part < 0 || part == 1) launch_acu_column(A, s);
+  if (A.fill && (part < 0 || part == 2)) {
+    HaloArgs H;
+    std::memset(&H, 0, sizeof(H));
+    H.g = A.g;
+    H.f[0] = A.ppdw;
+    H.f[1] = A.u;
+    H.f[2] = A.v;
+    H.f[3] = A.w;
+    H.nf = 4;
+    launch_halo(H, s);
+  }
+}
+
 void FusedStep::launch(Plan& P, std::vector<Op>& ops, StepDeps* deps) {
   const FusedData& D = *static_cast<FusedData*>(data);
   if (!deps) {
@@ -1758,22 +1775,19 @@ void FusedStep::launch_segment(Plan& P, std::vector<Op>& ops, int seg, int part)
   } else if (s.kind == kAdvect) {
     launch_adv(D.adv[s.aux[0]], s.aux[1], s.aux[2], P.stream);
   } else {
-    const AcuArgs& A = D.acu[s.aux[0]];
-    const Dims& g = A.g;
-    if (part < 0 || part == 0) launch_acu_uv(A, P.stream);
-    if (part < 0 || part == 1) launch_acu_column(A, P.stream);
-    if (A.fill && (part < 0 || part == 2)) {
-      HaloArgs H;
-      std::memset(&H, 0, sizeof(H));
-      H.g = g;
-      H.f[0] = A.ppdw;
-      H.f[1] = A.u;
-      H.f[2] = A.v;
-      H.f[3] = A.w;
-      H.nf = 4;
-      launch_halo(H, P.stream);
-    }
+    launch_substep(D.acu[s.aux[0]], part, P.stream);
   }
+}
+
+void FusedStep::play_segment(Plan& P, std::vector<Op>& ops, int seg, int part) {
+  const FusedSegment& s = segs.at(seg);
+  if (s.kind != kAcoustic || part >= 0) return launch_segment(P, ops, seg, part);
+  AcuArgs A = static_cast<FusedData*>(data)->acu[s.aux[0]];
+  A.ui = A.u = ops[s.first].args.p[6];
+  A.vi = A.v = ops[s.first].args.p[7];
+  A.wrap = 0;
+  A.fill = 1;
+  launch_substep(A, -1, P.stream);
 }
 
 int FusedStep::kernels(int seg) const {

@@ -30,6 +30,9 @@ struct FusedStep {
   void launch(Plan& P, std::vector<Op>& ops, StepDeps* deps);
   // one segment; part = -1 for all of its kernels, else the index of one of them
   void launch_segment(Plan& P, std::vector<Op>& ops, int seg, int part);
+  // the same for a caller that plays a segment on its own: a whole substep then starts from and
+  // ends in its fields, halos filled, wherever it stands in a run of them
+  void play_segment(Plan& P, std::vector<Op>& ops, int seg, int part);
   int kernels(int seg) const;  // launches of a fused segment (0: a run of exact ops)
   void release();
 };

@@ -700,7 +700,7 @@ int te_run_segment(te_ctx* ctx, int seg, int part) {
     P.fused_dirty = false;
   }
   if (seg < 0 || seg >= (int)P.fused.segs.size()) throw te::ApiError(TE_EINVAL, "segment out of range");
-  P.fused.launch_segment(P, P.active->ops, seg, part);
+  P.fused.play_segment(P, P.active->ops, seg, part);
   CU(cudaGetLastError());
   API_END(ctx)
 }
