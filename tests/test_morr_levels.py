@@ -36,6 +36,33 @@ def test_gpu_column_equals_the_host_build(variant, seed, nx, ny, nz):
 
 
 @pytest.mark.gpu
+def test_more_levels_in_device_memory_than_planned():
+    """nz of the device's parameter struct raised behind the host's copy (half a word written): the
+    column keeps to the planned levels."""
+    import ctypes
+    from thunderengine_web_b200.replayer import Replayer
+    cpu, op, M0 = morr_case('random', 1)
+    nz = int(M0[op.bind[0] + 2])
+    M0[op.bind[0]:op.bind[0] + 2] = np.array([50, 9], np.uint32)
+    cpu.M = M0.copy()
+    cpu.run(host_kernels().get, ops=[op])
+    tape, _, _, _ = helpers.load_golden_scenario('single_cell')
+    r = Replayer(tape, helpers.kernels_meta())
+    r.plan(False)
+    r.build()
+    r.write_words(0, M0[:r.buffers_end])
+    for w, n in ((op.bind[19], 1), (op.bind[0], 127)):   # dorad and the parameter struct
+        r.write_words(w, M0[w:w + n])
+    low = (ctypes.c_uint16 * 1)(nz + 24)
+    r._check(r.lib.te_write_words(r.h, int(op.bind[0]) + 2, low, 2))
+    oi = [k for k, o in enumerate(cpu.ops) if o is op][0]
+    r.run_ops(oi, oi)
+    got = r.read(r.buffers_end)
+    r.close()
+    assert np.array_equal(got, cpu.M[:r.buffers_end])
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize('nx,ny,nz', [(50, 9, 40), (33, 5, 9)])
 def test_gpu_reflectivity_equals_the_host_build(nx, ny, nz):
     from thunderengine_web_b200.replayer import Replayer

@@ -2412,7 +2412,9 @@ __global__ void __launch_bounds__(kMorrCols* kMorrWarps) k_morr_column(KArgs A, 
   const int t = blockIdx.x * kMorrCols + lane, ncol = A.gx * rows;
   const int i = t % A.gx, j = y0 + t / A.gx;
   const bool col = t < ncol && j < A.gy && i < p.nx && j < p.ny;
-  const int nk = p.nz, dorad = A.iv[19];
+  // the shared arrays hold the levels of the host's copy of the dimensions, whatever the device's
+  // words say since (written through te_device_ptr, or a part of a word)
+  const int nk = min(p.nz, A.g.nz), dorad = A.iv[19];
   const float DT = p.dt;
   morr::Fields F;
   F.T3 = A.p[1];
