@@ -62,7 +62,9 @@ int te_create(const te_config *cfg, te_ctx **out);
 
 /* Replayer.plan(withHashes) + Replayer.build() (replay.js:46-66, 180-209): lay out the
  * word memory for `tape_json`, allocate it on the device, write the setBytes payloads
- * and prepare the dispatch list of tape.steps[0].  `kernels_json` is the reference's
+ * and prepare the dispatch list of tape.steps[0].  Beyond mem_words, a step with runs of acoustic
+ * substeps gets two fields (2 x fieldStride bytes) of workspace if the device has room for
+ * them; its results are the same without.  `kernels_json` is the reference's
  * kernels.json (parameter ABI per kernel; NULL = the built-in table of this library). */
 int te_plan(te_ctx *ctx, const char *tape_json, size_t tape_len, const char *kernels_json,
             size_t kernels_len, int with_hashes);

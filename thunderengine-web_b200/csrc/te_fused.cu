@@ -1499,6 +1499,14 @@ static void chain_substeps(const Plan& P, std::vector<FusedSegment>& segs, std::
   }
 }
 
+bool FusedStep::chains_substeps(const std::vector<Op>& ops) {
+  FusedSegment s;
+  AcuArgs A;
+  for (size_t i = 0; i + 13 < ops.size(); i++)
+    if (match_substep(ops, i, s, A) && match_substep(ops, i + 13, s, A)) return true;
+  return false;
+}
+
 // What a fused phase leaves out: the output `out` of op `op`.
 struct Skipped {
   int op;

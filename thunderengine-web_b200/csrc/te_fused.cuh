@@ -33,6 +33,7 @@ struct FusedStep {
   // the same for a caller that plays a segment on its own: a whole substep then starts from and
   // ends in its fields, halos filled, wherever it stands in a run of them
   void play_segment(Plan& P, std::vector<Op>& ops, int seg, int part);
+  static bool chains_substeps(const std::vector<Op>& ops);  // a run of substeps that wants Plan::work
   int kernels(int seg) const;  // launches of a fused segment (0: a run of exact ops)
   void release();
 };

@@ -406,6 +406,18 @@ void Plan::finalize_args(std::vector<Op>& ops) {
   }
 }
 
+// Runs of substeps pass u and v through two more fields (te_fused.cu, K1).  Where the word memory
+// left no room for them every substep works in place.
+void Plan::reserve_workspace() {
+  if (work || !field_stride || !FusedStep::chains_substeps(active->ops)) return;
+  if (cudaMalloc(&work, 2 * field_stride) != cudaSuccess) {
+    cudaGetLastError();
+    work = nullptr;
+    return;
+  }
+  CU(cudaMemsetAsync(work, 0, 2 * field_stride, stream));
+}
+
 }  // namespace te
 
 // ------------------------------------------------------------------ C ABI
@@ -457,9 +469,7 @@ int te_plan(te_ctx* ctx, const char* tape_json, size_t tape_len, const char* ker
   P.release();
   P.load_kernel_meta(kernels_json, kernels_len);
   P.plan(tape_json, tape_len, with_hashes != 0);
-  // the word memory, then the fused steps' workspace: two fields (te_fused.cu, K1)
-  CU(cudaMalloc(&P.M, P.mem_words * 4 + 2 * P.field_stride));
-  P.work = P.field_stride ? reinterpret_cast<float*>(P.M + P.mem_words) : nullptr;
+  CU(cudaMalloc(&P.M, P.mem_words * 4));
   CU(cudaMemsetAsync(P.M, 0, P.mem_words * 4, ctx->plan.stream));
   CU(cudaMalloc(&P.H, std::max<size_t>(16, (size_t)P.hash_count * 4)));
   CU(cudaMemsetAsync(P.H, 0, std::max<size_t>(16, (size_t)P.hash_count * 4), ctx->plan.stream));
@@ -470,6 +480,7 @@ int te_plan(te_ctx* ctx, const char* tape_json, size_t tape_len, const char* ker
   P.finalize_args(P.active->ops);
   P.finalize_args(P.diag_ops);
   P.fused_dirty = P.exact_dirty = true;
+  P.reserve_workspace();
   API_END(ctx)
 }
 
@@ -552,6 +563,7 @@ int te_use_step(te_ctx* ctx, const char* cmds_json, size_t len) {
   if (cmds.type != te::JValue::Arr) throw te::ApiError(TE_EINVAL, "step must be a JSON array of commands");
   std::string sig = te::signature(cmds);
   auto it = P.cache.find(sig);
+  bool fresh = false;
   if (it == P.cache.end()) {
     te::Step st;
     st.offs = P.layout_bytes(cmds);
@@ -564,6 +576,7 @@ int te_use_step(te_ctx* ctx, const char* cmds_json, size_t len) {
     }
     P.bytes_init.clear();
     it = P.cache.emplace(sig, std::move(st)).first;
+    fresh = true;
   }
   te::Step& e = it->second;
   bool changed = (&e != P.active);
@@ -586,6 +599,7 @@ int te_use_step(te_ctx* ctx, const char* cmds_json, size_t len) {
     P.finalize_args(P.active->ops);
     P.invalidate_graphs();
   }
+  if (fresh) P.reserve_workspace();
   API_END(ctx)
 }
 
@@ -907,6 +921,7 @@ void Plan::release() {
   exact_fused.release();
   if (M) cudaFree(M);
   if (H) cudaFree(H);
+  if (work) cudaFree(work);
   M = nullptr;
   H = nullptr;
   work = nullptr;

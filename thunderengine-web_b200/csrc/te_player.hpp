@@ -78,7 +78,7 @@ struct Plan {
   // device
   uint32_t* M = nullptr;
   uint32_t* H = nullptr;
-  float* work = nullptr;  // two fields of workspace behind the word memory (no part of it)
+  float* work = nullptr;  // two fields of workspace for runs of substeps (none: they work in place)
   cudaGraphExec_t graph_exec = nullptr;
   cudaGraphExec_t graph_chain = nullptr;  // the chain a concurrent graph_exec replaced, which may still run
   int graph_runs = 0;             // steps launched since the step, mode or parameters last changed
@@ -94,6 +94,7 @@ struct Plan {
   std::vector<Op> build_ops(const JValue& cmds, const std::map<int, uint64_t>& offs, bool hashes);
   void plan(const char* tj, size_t tl, bool with_hashes);
   void finalize_args(std::vector<Op>& ops);
+  void reserve_workspace();  // `work`, if the active step has runs of substeps
   // with `deps` (during a capture) each op waits only for the ops it depends on
   void launch_exact(std::vector<Op>& ops, int first, int last, bool hashes, StepDeps* deps = nullptr);
   Access access(const void* p, bool write) const;         // the tape region a field pointer names
