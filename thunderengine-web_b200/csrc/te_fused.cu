@@ -1600,8 +1600,6 @@ static bool plain_bindings(const Plan& P, const std::vector<Op>& ops, const Fuse
 // One B200, per step: exact 128x128x64 1.58 -> 1.26 ms, exact 12x10x8 280 -> 197 us; the
 // per-dispatch form spent the difference on launches and on writing and re-reading fluxes.
 static void keep_final_stores(const Plan& P, const std::vector<Op>& ops, std::vector<FusedSegment>& segs, const FusedData& D) {
-  std::vector<std::vector<Access>> acc;
-  for (const Op& o : ops) acc.push_back(P.accesses(o));
   auto stored_again = [&](const Skipped& k, int last) {
     const Op& w = ops[k.op];
     const Access f = P.access(k.out, true);
@@ -1610,7 +1608,7 @@ static void keep_final_stores(const Plan& P, const std::vector<Op>& ops, std::ve
     auto within = [](const FaceRange& a, const FaceRange& b) { return covers(b, a.ilo, a.ihi, a.jlo, a.jhi, a.klo, a.khi); };
     for (size_t q = (size_t)last + 1; q < ops.size(); q++) {
       int touches = 0;
-      for (const Access& a : acc[q]) touches += a.lo < f.hi && f.lo < a.hi;
+      for (const Access& a : ops[q].acc) touches += a.lo < f.hi && f.lo < a.hi;
       if (!touches) continue;
       const Op& o = ops[q];
       if (o.copy || !o.spec || touches > 1 || !same_dims(o.args.g, w.args.g)) return false;
@@ -1762,7 +1760,7 @@ void FusedStep::launch(Plan& P, std::vector<Op>& ops, StepDeps* deps) {
       for (float* f : {A.rru, A.rrv, A.rrw, A.div3d, A.divx})
         if (f) acc.push_back(P.access(f, true));
       run(acc, q, 0);
-      if (!A.rru) run(P.accesses(ops[s.first + 1]), q, 1);
+      if (!A.rru) run(ops[s.first + 1].acc, q, 1);
     }
     else
       for (int part = 0; part < 2 + D.acu[s.aux[0]].fill; part++) run(acu_accesses(P, D.acu[s.aux[0]], part), q, part);

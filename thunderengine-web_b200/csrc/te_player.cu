@@ -279,6 +279,7 @@ void Plan::plan(const char* tj, size_t tl, bool with_hashes_) {
 
 void Plan::finalize_args(std::vector<Op>& ops) {
   for (Op& o : ops) {
+    if (o.copy) o.acc = regions(o);
     if (o.copy || !o.spec) continue;
     KArgs& A = o.args;
     std::memset(&A, 0, sizeof(A));
@@ -386,21 +387,26 @@ void Plan::finalize_args(std::vector<Op>& ops) {
       const uint64_t top = o.bind.at(1) + (gi - 1) + (uint64_t)A.g.sJ * ((gj - 1) + (uint64_t)A.g.sK * (gk - 1));
       if (gi && gj && gk && top >= mem_words) throw ApiError(TE_ERANGE, o.name + ": dispatch writes past the planned memory");
     }
+    if (o.name == "turb_zero") o.acc = regions(o);  // its extent depends on the dimensions
+    if (o.bound) continue;
+    // what follows from the bindings alone is the same for every payload of the step
+    o.bound = true;
+    o.acc = regions(o);
     // the __restrict__ build is valid when no written region overlaps another bound region
-    bool disjoint = true;
-    for (int q1 = 0; q1 < o.spec->nparams && disjoint; q1++) {
-      const ParamSpec& a = o.spec->params[q1];
-      auto ia = o.bind.find(a.index);
-      if (a.kind != kPtr || ia == o.bind.end()) continue;
-      const uint64_t a0 = ia->second, a1 = a0 + region_len(a0);
-      for (int q2 = q1 + 1; q2 < o.spec->nparams && disjoint; q2++) {
-        const ParamSpec& b = o.spec->params[q2];
-        auto ib = o.bind.find(b.index);
-        if (b.kind != kPtr || ib == o.bind.end() || !(a.write || b.write)) continue;
-        const uint64_t b0 = ib->second, b1 = b0 + region_len(b0);
-        if (a0 < b1 && b0 < a1) disjoint = false;
-      }
+    struct Bound {
+      uint64_t lo, hi;
+      bool write;
+    };
+    std::vector<Bound> ptrs;
+    for (int q = 0; q < o.spec->nparams; q++) {
+      const ParamSpec& ps = o.spec->params[q];
+      auto it = o.bind.find(ps.index);
+      if (ps.kind == kPtr && it != o.bind.end()) ptrs.push_back({it->second, it->second + region_len(it->second), ps.write != 0});
     }
+    bool disjoint = true;
+    for (size_t q1 = 0; q1 < ptrs.size() && disjoint; q1++)
+      for (size_t q2 = q1 + 1; q2 < ptrs.size() && disjoint; q2++)
+        disjoint = !((ptrs[q1].write || ptrs[q2].write) && ptrs[q1].lo < ptrs[q2].hi && ptrs[q2].lo < ptrs[q1].hi);
     const KernelSpec* f = disjoint ? fast::find_kernel(o.spec->name) : nullptr;
     o.launch = f ? f->launch : o.spec->launch;
   }
@@ -797,7 +803,7 @@ Access Plan::access(const void* p, bool write) const {
   return access_words(p, off < mem_words ? region_len(off) : field_stride / 4, write);  // a field of the workspace
 }
 
-std::vector<Access> Plan::accesses(const Op& o) const {
+std::vector<Access> Plan::regions(const Op& o) const {
   std::vector<Access> acc;
   if (o.copy) {
     acc.push_back(access_words(M + o.src, o.n, false));
@@ -828,7 +834,7 @@ void Plan::launch_exact(std::vector<Op>& ops, int first, int last, bool hashes, 
     Op& o = ops[i];
     if (deps) {
       if (!o.copy && !o.spec) throw ApiError(TE_ENOKERNEL, "no CUDA kernel for " + o.name);
-      CU(deps->run(accesses(o), [&] { launch_exact(ops, i, i, false); }));
+      CU(deps->run(o.acc, [&] { launch_exact(ops, i, i, false); }));
       continue;
     }
     if (o.copy) {

@@ -31,6 +31,8 @@ struct Op {
   std::map<int, uint64_t> bind;  // binding index -> memory word offset
   std::vector<HashReq> hashes;
   KArgs args;
+  std::vector<Access> acc;  // the words it reads and writes (Plan::regions)
+  bool bound = false;       // launch and acc, which follow from the bindings, are set
   short tile[2] = {0, 0};  // thread-block shape chosen by te_autotune (0: the launcher's default)
   uint64_t tile_y = 0;     // dispatch rows per scratch tile (replay.js:104-108)
 };
@@ -98,7 +100,7 @@ struct Plan {
   // with `deps` (during a capture) each op waits only for the ops it depends on
   void launch_exact(std::vector<Op>& ops, int first, int last, bool hashes, StepDeps* deps = nullptr);
   Access access(const void* p, bool write) const;         // the tape region a field pointer names
-  std::vector<Access> accesses(const Op& o) const;        // the words one op reads and writes
+  std::vector<Access> regions(const Op& o) const;         // the words one op reads and writes
   void launch_step_graph();
   // the active step (current mode) as a graph, not instantiated: a chain of its launches in
   // tape order or, concurrent, with the orders their data needs (te_deps.hpp)
