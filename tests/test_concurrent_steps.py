@@ -43,6 +43,20 @@ def test_synthetic_steps_equal_the_ops_in_tape_order(dims, moist, align, mode):
             assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), name
 
 
+# A tape may leave the field stride 0: the regions of its fields are then their grid's
+@pytest.mark.gpu
+@pytest.mark.parametrize('mode', [0, 1])
+def test_steps_of_a_tape_without_a_field_stride(mode):
+    run = timestep.Run(scenario.tiny(37, 29, 13, dx=500.0, dz=250.0, dt=3.0, nsound=8, us=25.0))
+    tape = run.tape(1)
+    tape['fieldStride'] = 0
+    (graph, ops), base = _both(tape, run.initial_buffers(), mode)
+    for name in run.fields:
+        if mode == 0 or name not in helpers.SCRATCH:
+            a, b = (helpers.field_view(m, run, base[run.rec.ids['arena']], name) for m in (graph, ops))
+            assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), name
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize('mode', [0, 1])
 @pytest.mark.parametrize('name', ['single_cell', 'squall_line'])

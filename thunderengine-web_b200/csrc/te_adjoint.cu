@@ -704,8 +704,8 @@ void reverse_step(Plan& P, AdjointState& S, StepDeps* deps) {
   std::vector<Op>& ops = P.active->ops;
   uint64_t cur = S.step_undo_words;
   auto adjoint_of = [&](const float* f, bool add) {
-    const uint64_t off = (uint64_t)(reinterpret_cast<const uint32_t*>(f) - P.M);
-    Access a = access_words(S.L + off, P.region_len(off), !add);
+    const Access of = P.access(f, !add);
+    Access a = access_words(S.L + (reinterpret_cast<const uint32_t*>(f) - P.M), (of.hi - of.lo) / 4, !add);
     a.add = add;
     return a;
   };

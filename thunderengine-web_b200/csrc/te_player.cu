@@ -239,6 +239,7 @@ void Plan::plan(const char* tj, size_t tl, bool with_hashes_) {
   buffers.clear();
   for (auto& b : tape.at("buffers").arr) buffers.push_back({(uint64_t)b.at("length").i64(), b.get("arena") && b.at("arena").truthy()});
   field_stride = (uint64_t)tape.at("fieldStride").i64();
+  field_words = field_stride / 4;
   uint64_t top = 0;
   base.clear();
   for (auto& b : buffers) {
@@ -279,7 +280,6 @@ void Plan::plan(const char* tj, size_t tl, bool with_hashes_) {
 
 void Plan::finalize_args(std::vector<Op>& ops) {
   for (Op& o : ops) {
-    if (o.copy) o.acc = regions(o);
     if (o.copy || !o.spec) continue;
     KArgs& A = o.args;
     std::memset(&A, 0, sizeof(A));
@@ -323,6 +323,7 @@ void Plan::finalize_args(std::vector<Op>& ops) {
       uint64_t count = ok ? (uint64_t)g.sJ * g.sK * (g.nz + 1) : 0;
       ok = ok && count < (1ull << 31) && (field_stride == 0 || count * 4 <= field_stride);
       if (!ok) throw ApiError(TE_EINVAL, o.name + ": GridDims out of range or larger than the arena field stride");
+      field_words = std::max(field_words, count);
     }
     if (o.spec->acoustic) {
       auto it1 = o.bind.find(1);
@@ -387,11 +388,12 @@ void Plan::finalize_args(std::vector<Op>& ops) {
       const uint64_t top = o.bind.at(1) + (gi - 1) + (uint64_t)A.g.sJ * ((gj - 1) + (uint64_t)A.g.sK * (gk - 1));
       if (gi && gj && gk && top >= mem_words) throw ApiError(TE_ERANGE, o.name + ": dispatch writes past the planned memory");
     }
-    if (o.name == "turb_zero") o.acc = regions(o);  // its extent depends on the dimensions
-    if (o.bound) continue;
+  }
+  for (Op& o : ops) {
+    if (o.copy || (o.spec && (!o.bound || o.name == "turb_zero"))) o.acc = regions(o);  // turb_zero's extent depends on nz
+    if (o.copy || !o.spec || o.bound) continue;
     // what follows from the bindings alone is the same for every payload of the step
     o.bound = true;
-    o.acc = regions(o);
     // the __restrict__ build is valid when no written region overlaps another bound region
     struct Bound {
       uint64_t lo, hi;
@@ -800,7 +802,13 @@ namespace te {
 
 Access Plan::access(const void* p, bool write) const {
   const uint64_t off = (uint64_t)(static_cast<const uint32_t*>(p) - M);
-  return access_words(p, off < mem_words ? region_len(off) : field_stride / 4, write);  // a field of the workspace
+  if (off >= mem_words) return access_words(p, field_words, write);  // a field of the workspace
+  uint64_t len = region_len(off);
+  if (!len && off < buffers_end) {  // in the arena of a tape without a field stride
+    const size_t n = std::upper_bound(base.begin(), base.end(), off) - base.begin();
+    len = std::min(field_words, base[n - 1] + buffers[n - 1].length / 4 - off);
+  }
+  return access_words(p, len, write);
 }
 
 std::vector<Access> Plan::regions(const Op& o) const {

@@ -68,6 +68,7 @@ struct Plan {
   std::vector<BufInfo> buffers;
   std::vector<uint64_t> base;
   uint64_t field_stride = 0;  // bytes
+  uint64_t field_words = 0;   // words of a field: the stride's, or without one the largest grid's
   uint64_t buffers_end = 0, bytes_top = 0, bytes_spare_end = 0, scratch_base = 0, scratch_need = 0, mem_words = 0;
   uint32_t hash_count = 0;
   bool with_hashes = false;
