@@ -43,6 +43,47 @@ def test_synthetic_steps_equal_the_ops_in_tape_order(dims, moist, align, mode):
             assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), name
 
 
+# A refused change of parameters leaves the step as it was, also for the graph that is built later
+@pytest.mark.gpu
+@pytest.mark.parametrize('how', ['step', 'words'])
+def test_a_refused_change_of_parameters(how):
+    import base64
+    import copy
+    import struct
+    run = timestep.Run(scenario.tiny(12, 10, 8, dx=500.0, dz=250.0, dt=3.0, nsound=8, us=25.0))
+    tape = run.tape(1)
+    init = run.initial_buffers()
+    (want, _), _ = _both(tape, init, 0)
+    r = helpers.gpu_replayer(tape, init, hashes=False)
+    r.encode_steps(4)
+    step = copy.deepcopy(tape['steps'][0])
+    dims = [c for c in step if c['op'] == 'bytes' and c['index'] == 0][40]   # of a dispatch amid the step
+    raw = base64.b64decode(dims['data'])
+    with pytest.raises(RuntimeError, match='GridDims'):
+        if how == 'step':
+            dims['data'] = base64.b64encode(struct.pack('<i', 0) + raw[4:]).decode()
+            r.use_step(step)
+        else:
+            r.write_words(_payload_offset(tape, step, dims), np.zeros(1, np.uint32))
+    r.encode_steps(STEPS - 4)
+    assert np.array_equal(r.read(r.buffers_end), want)
+    r.close()
+
+
+def _payload_offset(tape, step, cmd):
+    """Word offset of the parameter words of a setBytes command (its place among them)."""
+    from oracle.player import CpuPlayer
+    p = CpuPlayer(tape, helpers.kernels_meta())
+    p.plan(False)
+    at = p.buffers_end
+    for c in step:
+        if c is cmd:
+            return at
+        if c['op'] == 'bytes':
+            import base64
+            at += -(-(-(-len(base64.b64decode(c['data'])) // 4)) // 4) * 4 + 4
+
+
 # A tape may leave the field stride 0: the regions of its fields are then their grid's
 @pytest.mark.gpu
 @pytest.mark.parametrize('mode', [0, 1])

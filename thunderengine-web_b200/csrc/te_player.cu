@@ -278,11 +278,14 @@ void Plan::plan(const char* tj, size_t tl, bool with_hashes_) {
   for (auto& bi : bytes_init) std::memcpy(&host_bytes[bi.first - buffers_end], bi.second.data(), bi.second.size());
 }
 
+// Throws on a parameter it refuses and then leaves every op's arguments as they were: the step may
+// still be played, and captured again (launch_step_graph), with those.
 void Plan::finalize_args(std::vector<Op>& ops) {
-  for (Op& o : ops) {
+  std::vector<KArgs> args(ops.size());  // zeroed
+  for (size_t i = 0; i < ops.size(); i++) {
+    const Op& o = ops[i];
     if (o.copy || !o.spec) continue;
-    KArgs& A = o.args;
-    std::memset(&A, 0, sizeof(A));
+    KArgs& A = args[i];
     A.bx = o.tile[0];
     A.by = o.tile[1];
     A.gx = o.grid[0];
@@ -389,6 +392,8 @@ void Plan::finalize_args(std::vector<Op>& ops) {
       if (gi && gj && gk && top >= mem_words) throw ApiError(TE_ERANGE, o.name + ": dispatch writes past the planned memory");
     }
   }
+  for (size_t i = 0; i < ops.size(); i++)
+    if (!ops[i].copy && ops[i].spec) ops[i].args = args[i];
   for (Op& o : ops) {
     if (o.copy || (o.spec && (!o.bound || o.name == "turb_zero"))) o.acc = regions(o);  // turb_zero's extent depends on nz
     if (o.copy || !o.spec || o.bound) continue;
@@ -529,8 +534,8 @@ int te_write_words(te_ctx* ctx, uint64_t word_off, const void* data, size_t byte
   if (lo < hi) {
     std::memcpy(&P.host_bytes[lo - P.buffers_end], (const uint8_t*)data + (lo - word_off) * 4, (hi - lo) * 4);
     P.finalize_args(P.active->ops);
-    P.finalize_args(P.diag_ops);
     P.invalidate_graphs();
+    P.finalize_args(P.diag_ops);
   }
   API_END(ctx)
 }
@@ -588,25 +593,42 @@ int te_use_step(te_ctx* ctx, const char* cmds_json, size_t len) {
   }
   te::Step& e = it->second;
   bool changed = (&e != P.active);
+  // the payloads are checked with the host's copy first; a refused one leaves the active step,
+  // its arguments and the device's words as they were
+  struct Payload {
+    int cmd;
+    uint64_t off;
+    std::vector<uint8_t> words, old;
+  };
+  std::vector<Payload> payloads;
   for (size_t i = 0; i < cmds.arr.size(); i++) {
     const te::JValue& c = cmds.arr[i];
     if (c.at("op").str != "bytes") continue;
     auto d = e.data.find((int)i);
     if (d != e.data.end() && d->second == c.at("data").str) continue;
-    e.data[(int)i] = c.at("data").str;
-    std::vector<uint8_t> raw = te::base64_decode(c.at("data").str);
-    raw.resize(te::ceil_div(raw.size(), 4) * 4, 0);
-    uint64_t off = e.offs.at((int)i);
-    std::memcpy(&P.host_bytes[off - P.buffers_end], raw.data(), raw.size());
-    CU(cudaMemcpyAsync(P.M + off, raw.data(), raw.size(), cudaMemcpyHostToDevice, ctx->plan.stream));
+    Payload p{(int)i, e.offs.at((int)i), te::base64_decode(c.at("data").str), {}};
+    p.words.resize(te::ceil_div(p.words.size(), 4) * 4, 0);
+    uint8_t* host = reinterpret_cast<uint8_t*>(&P.host_bytes[p.off - P.buffers_end]);
+    p.old.assign(host, host + p.words.size());
+    std::memcpy(host, p.words.data(), p.words.size());
+    payloads.push_back(std::move(p));
     changed = true;
+  }
+  if (changed) {
+    try {
+      P.finalize_args(e.ops);
+    } catch (...) {
+      for (const Payload& p : payloads) std::memcpy(&P.host_bytes[p.off - P.buffers_end], p.old.data(), p.old.size());
+      throw;
+    }
+  }
+  for (const Payload& p : payloads) {
+    e.data[p.cmd] = cmds.arr[p.cmd].at("data").str;
+    CU(cudaMemcpyAsync(P.M + p.off, p.words.data(), p.words.size(), cudaMemcpyHostToDevice, ctx->plan.stream));
   }
   CU(cudaStreamSynchronize(ctx->plan.stream));
   P.active = &e;
-  if (changed) {
-    P.finalize_args(P.active->ops);
-    P.invalidate_graphs();
-  }
+  if (changed) P.invalidate_graphs();
   if (fresh) P.reserve_workspace();
   API_END(ctx)
 }
