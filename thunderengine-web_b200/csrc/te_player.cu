@@ -281,11 +281,13 @@ void Plan::plan(const char* tj, size_t tl, bool with_hashes_) {
 // Throws on a parameter it refuses and then leaves every op's arguments as they were: the step may
 // still be played, and captured again (launch_step_graph), with those.
 void Plan::finalize_args(std::vector<Op>& ops) {
-  std::vector<KArgs> args(ops.size());  // zeroed
+  std::vector<KArgs>& args = new_args;
+  if (args.size() < ops.size()) args.resize(ops.size());
   for (size_t i = 0; i < ops.size(); i++) {
     const Op& o = ops[i];
     if (o.copy || !o.spec) continue;
     KArgs& A = args[i];
+    std::memset(&A, 0, sizeof(A));
     A.bx = o.tile[0];
     A.by = o.tile[1];
     A.gx = o.grid[0];
