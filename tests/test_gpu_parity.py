@@ -386,16 +386,21 @@ def test_fused_tall_columns_vs_oracle(nz):
 
 
 def test_headline_config_fused_equals_exact_over_20_steps():
-    """20 large steps at 256x256x80 in fused and in exact mode on the GPU: every
-    non-scratch field bit-identical."""
+    """20 large steps at 256x256x80 in fused and in exact mode on the GPU against the same steps played
+    one kernel per dispatch: every non-scratch field (exact mode: every word) bit-identical."""
     from thunderengine_web_b200.replayer import TE_MODE_FUSED
     run = timestep.Run(scenario.AT_SCALE)
     tape = run.tape(1)
     init = run.initial_buffers()
     ex = helpers.gpu_replayer(tape, init, hashes=False)
-    ex.encode_steps(20)
+    for _ in range(20):
+        ex.run_ops(0, ex.num_ops - 1)
     mem_ex = ex.read(ex.buffers_end)
     base = ex.base[run.rec.ids['arena']]
+    ex.close()
+    ex = helpers.gpu_replayer(tape, init, hashes=False)
+    ex.encode_steps(20)
+    assert np.array_equal(ex.read(ex.buffers_end), mem_ex)
     ex.close()
     fz = helpers.gpu_replayer(tape, init, hashes=False, mode=TE_MODE_FUSED)
     fz.encode_steps(20)
@@ -409,8 +414,8 @@ def test_headline_config_fused_equals_exact_over_20_steps():
 
 def test_large_domain_step_fused_equals_exact():
     """1024x1024x100 (dx 250 m, dt 1.5 s, nsound 8, three-bubble line): ~21 GB of arena,
-    word offsets past 2^32.  One step in fused and in exact mode: every non-scratch field
-    bit-identical, finite, and the state moved."""
+    word offsets past 2^32.  One step in fused mode and one kernel per dispatch: every non-scratch
+    field bit-identical, finite, and the state moved."""
     import psutil
     from thunderengine_web_b200.replayer import Replayer, TE_MODE_FUSED
     if psutil.virtual_memory().available < 64 << 30:
@@ -430,7 +435,10 @@ def test_large_domain_step_fused_equals_exact():
                 r.upload(b['id'], run.buffer_bytes(b['label']))
         r.write_words(r.base[aid], arena)
         r.set_mode(mode)
-        r.encode_steps(1)
+        if mode:
+            r.encode_steps(1)
+        else:
+            r.run_ops(0, r.num_ops - 1)
         r.sync()
         reps.append(r)
     g = run.grid
@@ -509,29 +517,33 @@ def test_recorded_step_in_fused_mode_equals_exact():
     """The single_cell recording (open lateral boundaries, full physics) in fused mode: the
     planner fuses the advection of every variable there (with adv_assemble's open-edge
     branches) and runs the rest per dispatch; after one step every field but the step
-    scratch equals the exact-mode step, word for word."""
+    scratch, and in exact mode every word, equals the step played one kernel per dispatch."""
     from thunderengine_web_b200.replayer import Replayer, TE_MODE_FUSED
     tape, init, _, _ = helpers.load_golden_scenario('single_cell')
     km = helpers.kernels_meta()
     mems = []
-    for mode in (0, TE_MODE_FUSED):
+    for mode in (None, 0, TE_MODE_FUSED):
         r = Replayer(tape, km)
         r.plan(False)
         r.build()
         for i, b in init.items():
             r.upload(i, b)
-        r.set_mode(mode)
+        r.set_mode(mode or 0)
         if mode:
             segs = r.fused_segments()
             assert sum(1 for s in segs if s[0] == 3) >= 10   # the advection phases are fused
-        r.encode_steps(1)
+        if mode is None:
+            r.run_ops(0, r.num_ops - 1)
+        else:
+            r.encode_steps(1)
         mems.append(r.read(r.buffers_end))
         base = r.base[2]
         r.close()
+    assert np.array_equal(mems[1], mems[0])
     for name, off in tape['fields'].items():
         if name in STEP_SCRATCH:
             continue
         n = (tape['nx'] + 7) * (tape['ny'] + 7) * (tape['nz'] + 1)
         a = mems[0][base + off // 4:base + off // 4 + n]
-        b = mems[1][base + off // 4:base + off // 4 + n]
+        b = mems[2][base + off // 4:base + off // 4 + n]
         assert np.array_equal(a, b), name
