@@ -1499,11 +1499,18 @@ static void chain_substeps(const Plan& P, std::vector<FusedSegment>& segs, std::
   }
 }
 
+// By the ops' names alone, before their arguments are known.
 bool FusedStep::chains_substeps(const std::vector<Op>& ops) {
-  FusedSegment s;
-  AcuArgs A;
-  for (size_t i = 0; i + 13 < ops.size(); i++)
-    if (match_substep(ops, i, s, A) && match_substep(ops, i + 13, s, A)) return true;
+  auto substep = [&](size_t i) {
+    if (i + 13 > ops.size()) return false;
+    for (int q = 0; q < 4; q++)
+      if (!is_name(ops[i + q], kSubstep[q])) return false;
+    for (int q : {4, 7, 9, 11})
+      if (!is_name(ops[i + q], "bc_periodic_x")) return false;
+    return true;
+  };
+  for (size_t i = 0; i < ops.size(); i++)
+    if (substep(i) && substep(i + 13)) return true;
   return false;
 }
 
@@ -1603,8 +1610,8 @@ static void keep_final_stores(const Plan& P, const std::vector<Op>& ops, std::ve
   auto stored_again = [&](const Skipped& k, int last) {
     const Op& w = ops[k.op];
     const Access f = P.access(k.out, true);
-    FaceRange skipped, r, own{0, -1, 0, -1, 0, -1};  // own: faces written since
-    const bool flux = flux_store(w, k.out, skipped);
+    FaceRange r, own{0, -1, 0, -1, 0, -1};  // own: faces written since
+    const bool flux = flux_store(w, k.out, r);
     auto within = [](const FaceRange& a, const FaceRange& b) { return covers(b, a.ilo, a.ihi, a.jlo, a.jhi, a.klo, a.khi); };
     for (size_t q = (size_t)last + 1; q < ops.size(); q++) {
       int touches = 0;
@@ -1615,7 +1622,6 @@ static void keep_final_stores(const Plan& P, const std::vector<Op>& ops, std::ve
       // its one binding on the field is the output (adv_assemble's accumulation reads it)
       if (same_store(o, w, k.out)) return !(o.name == "adv_assemble" && o.args.iv[12] != 0);
       if (flux && flux_store(o, k.out, r)) {
-        if (within(skipped, r)) return true;
         own = r;
       } else if (!(flux && faces_read(o, k.out, r) && within(r, own))) {
         return false;

@@ -422,14 +422,16 @@ void Plan::finalize_args(std::vector<Op>& ops) {
 }
 
 // Runs of substeps pass u and v through two more fields (te_fused.cu, K1).  Where the word memory
-// left no room for them every substep works in place.
+// left no room for them every substep works in place.  te_plan has made room for its step;
+// this is for a step structure that comes later.
 void Plan::reserve_workspace() {
   if (work || !field_stride || !FusedStep::chains_substeps(active->ops)) return;
-  if (cudaMalloc(&work, 2 * field_stride) != cudaSuccess) {
+  if (cudaMalloc(&work_own, 2 * field_stride) != cudaSuccess) {
     cudaGetLastError();
-    work = nullptr;
+    work_own = nullptr;
     return;
   }
+  work = work_own;
   CU(cudaMemsetAsync(work, 0, 2 * field_stride, stream));
 }
 
@@ -484,7 +486,16 @@ int te_plan(te_ctx* ctx, const char* tape_json, size_t tape_len, const char* ker
   P.release();
   P.load_kernel_meta(kernels_json, kernels_len);
   P.plan(tape_json, tape_len, with_hashes != 0);
-  CU(cudaMalloc(&P.M, P.mem_words * 4));
+  // one allocation for the word memory and, where the step wants it and there is room, the
+  // workspace behind it (a second one cost 3-5 ms)
+  const uint64_t bytes = P.mem_words * 4, more = te::FusedStep::chains_substeps(P.active->ops) ? 2 * P.field_stride : 0;
+  if (more && cudaMalloc(&P.M, bytes + more) == cudaSuccess) {
+    P.work = reinterpret_cast<float*>(P.M + P.mem_words);
+    CU(cudaMemsetAsync(P.work, 0, more, ctx->plan.stream));
+  } else {
+    cudaGetLastError();
+    CU(cudaMalloc(&P.M, bytes));
+  }
   CU(cudaMemsetAsync(P.M, 0, P.mem_words * 4, ctx->plan.stream));
   CU(cudaMalloc(&P.H, std::max<size_t>(16, (size_t)P.hash_count * 4)));
   CU(cudaMemsetAsync(P.H, 0, std::max<size_t>(16, (size_t)P.hash_count * 4), ctx->plan.stream));
@@ -495,7 +506,6 @@ int te_plan(te_ctx* ctx, const char* tape_json, size_t tape_len, const char* ker
   P.finalize_args(P.active->ops);
   P.finalize_args(P.diag_ops);
   P.fused_dirty = P.exact_dirty = true;
-  P.reserve_workspace();
   API_END(ctx)
 }
 
@@ -959,7 +969,8 @@ void Plan::release() {
   exact_fused.release();
   if (M) cudaFree(M);
   if (H) cudaFree(H);
-  if (work) cudaFree(work);
+  if (work_own) cudaFree(work_own);
+  work_own = nullptr;
   M = nullptr;
   H = nullptr;
   work = nullptr;

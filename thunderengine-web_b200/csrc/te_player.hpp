@@ -82,7 +82,8 @@ struct Plan {
   // device
   uint32_t* M = nullptr;
   uint32_t* H = nullptr;
-  float* work = nullptr;  // two fields of workspace for runs of substeps (none: they work in place)
+  float* work = nullptr;  // two fields of workspace for runs of substeps (none: they work in place),
+  float* work_own = nullptr;  // behind the word memory or an allocation of their own
   cudaGraphExec_t graph_exec = nullptr;
   cudaGraphExec_t graph_chain = nullptr;  // the chain a concurrent graph_exec replaced, which may still run
   int graph_runs = 0;             // steps launched since the step, mode or parameters last changed
