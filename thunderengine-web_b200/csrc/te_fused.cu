@@ -1548,28 +1548,37 @@ static bool same_store(const Op& o, const Op& w, const float* out) {
   return true;
 }
 
-// The faces a flux dispatch writes into `out`.
-static bool flux_store(const Op& o, const float* out, FaceRange& r) {
+// The faces a flux dispatch writes into `out`; it reads none of it (the caller has seen that the
+// op binds the field once).
+static bool faces_written(const Op& o, const float* out, FaceRange& r) {
   for (auto& fs : kFluxSets) {
     const int dir = o.name == fs.x ? 0 : o.name == fs.y ? 1 : o.name == fs.z ? 2 : -1;
     if (dir < 0) continue;
     r = flux_range(fs.kind, dir, o);
     return o.args.p[dir == 2 ? fs.out_z : fs.out_h] == out;
   }
-  return false;
+  if (o.name != "turb_scalar_flux_h") return false;
+  const Dims& g = o.args.g;
+  r = FaceRange{0, std::min(o.grid[0] - 1, g.nx), 0, std::min(o.grid[1] - 1, g.ny), 0, std::min(o.grid[2], g.nz) - 1};
+  return o.args.p[5] == out || o.args.p[6] == out;
 }
 
-// The faces of `out`, one of its three flux fields, that adv_assemble reads.
+// A box that holds the faces of `out` that an op on flux fields reads, and any it then writes.
 static bool faces_read(const Op& o, const float* out, FaceRange& r) {
-  if (o.name != "adv_assemble") return false;
   const Dims& g = o.args.g;
-  const int st = std::abs(o.args.iv[1]);
-  r = FaceRange{0, st == 2 ? g.nx : g.nx - 1, 0, st == 3 ? g.ny : g.ny - 1, st == 4 ? 1 : 0, g.nz - 1};
-  const int dir = out == o.args.p[3] ? 0 : out == o.args.p[4] ? 1 : out == o.args.p[5] ? 2 : -1;
-  if (dir == 0) (st == 2 ? r.ilo : r.ihi) += st == 2 ? -1 : 1;
-  if (dir == 1) (st == 3 ? r.jlo : r.jhi) += st == 3 ? -1 : 1;
-  if (dir == 2) (st == 4 ? r.klo : r.khi) += st == 4 ? -1 : 1;
-  return dir >= 0;
+  if (o.name == "adv_assemble") {
+    const int st = std::abs(o.args.iv[1]);
+    r = FaceRange{0, st == 2 ? g.nx : g.nx - 1, 0, st == 3 ? g.ny : g.ny - 1, st == 4 ? 1 : 0, g.nz - 1};
+    const int dir = out == o.args.p[3] ? 0 : out == o.args.p[4] ? 1 : out == o.args.p[5] ? 2 : -1;
+    if (dir == 0) (st == 2 ? r.ilo : r.ihi) += st == 2 ? -1 : 1;
+    if (dir == 1) (st == 3 ? r.jlo : r.jhi) += st == 3 ? -1 : 1;
+    if (dir == 2) (st == 4 ? r.klo : r.khi) += st == 4 ? -1 : 1;
+    return dir >= 0;
+  }
+  r = FaceRange{0, g.nx, 0, g.ny, 0, g.nz};
+  if (o.name == "turb_openbc_flux") return out == o.args.p[1] || out == o.args.p[2];
+  if (o.name == "turb_scalar_vert_implicit") return out == o.args.p[8] || out == o.args.p[9];
+  return false;
 }
 
 // What a phase writes, in its ops or its fused kernels, is a field of its own: no other binding
@@ -1601,18 +1610,17 @@ static bool plain_bindings(const Plan& P, const std::vector<Op>& ops, const Fuse
 // keep_scratch (exact mode): a phase stays fused when every store it skips is made again later in
 // the step, by a dispatch that writes (at least) the same words without reading the field, and
 // nothing reads them before that.  Flux dispatches in between may write a part of the field and
-// assemblies read back what those wrote.  The later dispatch runs, or is itself skipped for one
+// ops on fluxes read back what those wrote.  The later dispatch runs, or is itself skipped for one
 // that is later still, so every word ends with the value of its last writer.  Of a moist step the
-// last substep and the last variable of each flux kind run per dispatch (333 launches -> 124).
+// last substep and the last variable of each flux kind run per dispatch (333 launches -> 130).
 // One B200, per step: exact 128x128x64 1.58 -> 1.26 ms, exact 12x10x8 280 -> 197 us; the
 // per-dispatch form spent the difference on launches and on writing and re-reading fluxes.
 static void keep_final_stores(const Plan& P, const std::vector<Op>& ops, std::vector<FusedSegment>& segs, const FusedData& D) {
   auto stored_again = [&](const Skipped& k, int last) {
     const Op& w = ops[k.op];
     const Access f = P.access(k.out, true);
-    FaceRange r, own{0, -1, 0, -1, 0, -1};  // own: faces written since
-    const bool flux = flux_store(w, k.out, r);
-    auto within = [](const FaceRange& a, const FaceRange& b) { return covers(b, a.ilo, a.ihi, a.jlo, a.jhi, a.klo, a.khi); };
+    FaceRange r, skipped, own{0, -1, 0, -1, 0, -1};  // own: faces written since
+    const bool flux = faces_written(w, k.out, skipped);
     for (size_t q = (size_t)last + 1; q < ops.size(); q++) {
       int touches = 0;
       for (const Access& a : ops[q].acc) touches += a.lo < f.hi && f.lo < a.hi;
@@ -1621,9 +1629,12 @@ static void keep_final_stores(const Plan& P, const std::vector<Op>& ops, std::ve
       if (o.copy || !o.spec || touches > 1 || !same_dims(o.args.g, w.args.g)) return false;
       // its one binding on the field is the output (adv_assemble's accumulation reads it)
       if (same_store(o, w, k.out)) return !(o.name == "adv_assemble" && o.args.iv[12] != 0);
-      if (flux && flux_store(o, k.out, r)) {
+      if (flux && faces_written(o, k.out, r)) {
         own = r;
-      } else if (!(flux && faces_read(o, k.out, r) && within(r, own))) {
+      } else if (!flux || !faces_read(o, k.out, r) ||
+                 // the skipped faces among those it reads are written since
+                 !covers(own, std::max(r.ilo, skipped.ilo), std::min(r.ihi, skipped.ihi), std::max(r.jlo, skipped.jlo),
+                         std::min(r.jhi, skipped.jhi), std::max(r.klo, skipped.klo), std::min(r.khi, skipped.khi))) {
         return false;
       }
     }

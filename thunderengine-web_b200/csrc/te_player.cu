@@ -281,12 +281,12 @@ void Plan::plan(const char* tj, size_t tl, bool with_hashes_) {
 // Throws on a parameter it refuses and then leaves every op's arguments as they were: the step may
 // still be played, and captured again (launch_step_graph), with those.
 void Plan::finalize_args(std::vector<Op>& ops) {
-  std::vector<KArgs>& args = new_args;
-  if (args.size() < ops.size()) args.resize(ops.size());
+  std::vector<KArgs>& args = new_args;  // (a step without arguments yet is not played: in place)
   for (size_t i = 0; i < ops.size(); i++) {
-    const Op& o = ops[i];
+    Op& o = ops[i];
     if (o.copy || !o.spec) continue;
-    KArgs& A = args[i];
+    if (o.bound && args.size() < ops.size()) args.resize(ops.size());
+    KArgs& A = o.bound ? args[i] : o.args;
     std::memset(&A, 0, sizeof(A));
     A.bx = o.tile[0];
     A.by = o.tile[1];
@@ -395,18 +395,19 @@ void Plan::finalize_args(std::vector<Op>& ops) {
     }
   }
   for (size_t i = 0; i < ops.size(); i++)
-    if (!ops[i].copy && ops[i].spec) ops[i].args = args[i];
+    if (!ops[i].copy && ops[i].spec && ops[i].bound) ops[i].args = args[i];
+  struct Bound {
+    uint64_t lo, hi;
+    bool write;
+  };
+  std::vector<Bound> ptrs;
   for (Op& o : ops) {
     if (o.copy || (o.spec && (!o.bound || o.name == "turb_zero"))) o.acc = regions(o);  // turb_zero's extent depends on nz
     if (o.copy || !o.spec || o.bound) continue;
     // what follows from the bindings alone is the same for every payload of the step
     o.bound = true;
     // the __restrict__ build is valid when no written region overlaps another bound region
-    struct Bound {
-      uint64_t lo, hi;
-      bool write;
-    };
-    std::vector<Bound> ptrs;
+    ptrs.clear();
     for (int q = 0; q < o.spec->nparams; q++) {
       const ParamSpec& ps = o.spec->params[q];
       auto it = o.bind.find(ps.index);
@@ -853,6 +854,7 @@ std::vector<Access> Plan::regions(const Op& o) const {
     return acc;
   }
   if (!o.spec) return acc;
+  acc.reserve(o.spec->nparams);
   for (int q = 0; q < o.spec->nparams; q++) {
     const ParamSpec& ps = o.spec->params[q];
     const float* p = ps.index >= 0 && ps.index < kMaxBind ? o.args.p[ps.index] : nullptr;
