@@ -1422,24 +1422,28 @@ static std::vector<Access> halo_accesses(const Plan& P, const HaloArgs& H) {
   return acc;
 }
 
-static std::vector<Access> adv_reads(const Plan& P, const AdvArgs& A, int kind) {
-  std::vector<Access> acc;
+static std::vector<const float*> adv_reads(const AdvArgs& A, int kind) {
+  std::vector<const float*> f;
+  f.reserve(24);
+  auto add = [&](const float* p) {
+    if (p && std::find(f.begin(), f.end(), p) == f.end()) f.push_back(p);
+  };
   const FluxNames* fs = nullptr;
   for (auto& c : kFluxSets)
     if (c.kind == kind) fs = &c;
   for (int b = 0; b < kMaxBind; b++) {
-    if (b != fs->out_h && A.fx.p[b]) acc.push_back(P.access(A.fx.p[b], false));
-    if (b != fs->out_h && A.fy.p[b]) acc.push_back(P.access(A.fy.p[b], false));
-    if (b != fs->out_z && A.fz.p[b]) acc.push_back(P.access(A.fz.p[b], false));
-    if (b != 3 && b != 4 && b != 5 && b != 11 && b != 19 && A.as.p[b]) acc.push_back(P.access(A.as.p[b], false));
+    if (b != fs->out_h) add(A.fx.p[b]);
+    if (b != fs->out_h) add(A.fy.p[b]);
+    if (b != fs->out_z) add(A.fz.p[b]);
+    if (b != 3 && b != 4 && b != 5 && b != 11 && b != 19) add(A.as.p[b]);
   }
-  for (const float* f : {A.div3d, A.thterm, A.phiA})
-    if (f) acc.push_back(P.access(f, false));
-  return acc;
+  for (const float* p : {A.div3d, A.thterm, A.phiA}) add(p);
+  return f;
 }
 
 static std::vector<Access> adv_accesses(const Plan& P, const AdvArgs& A, int kind) {
-  std::vector<Access> acc = adv_reads(P, A, kind);
+  std::vector<Access> acc;
+  for (const float* f : adv_reads(A, kind)) acc.push_back(P.access(f, false));
   // an RK update that keeps its tendency to itself still reads it on open u, v edges
   acc.push_back(P.access(A.dest, A.accumulate || A.write_dest));
   for (float* f : {A.phi, A.fxo, A.fyo, A.fzo})
@@ -1597,7 +1601,7 @@ static bool plain_bindings(const Plan& P, const std::vector<Op>& ops, const Fuse
     const KArgs& as = ops[s.first + 3].args;
     wr = {A.dest, as.p[3], as.p[4], as.p[5]};
     if (A.phi) wr.push_back(A.phi);
-    for (const Access& a : adv_reads(P, A, s.aux[1])) rd.push_back(reinterpret_cast<const float*>(a.lo));
+    rd = adv_reads(A, s.aux[1]);
   } else if (s.kind == kHalo) {
     const HaloArgs& H = D.halo[s.aux[0]];
     wr.assign(H.f, H.f + H.nf);
