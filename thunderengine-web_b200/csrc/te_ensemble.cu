@@ -133,7 +133,12 @@ int te_ensemble_create(te_ctx* const* members, int n, te_ensemble** out) {
     ECU(cudaGraphCreate(&root, 0));
     try {
       for (te_ctx* c : E->members) {
-        cudaGraph_t g = c->plan.capture_step(false);  // the members already run side by side
+        // Chains: the members already run side by side, and the orders of many concurrent steps
+        // cost more than they give.  One B200, us a step, chains / concurrent: 12 members of about
+        // 24x20x16 467 / 803, 64 of them 1953 / 12349, 12 of 64x64x40 2736 / 3036; 3 of 128x128x64
+        // 3420 / 3388, of 256x256x80 15379 / 15565.  Two or three small members would gain
+        // (3 of 24x20x16 378 / 288, of 64x64x40 777 / 712).
+        cudaGraph_t g = c->plan.capture_step(false);
         cudaGraphNode_t node;
         const cudaError_t e = cudaGraphAddChildGraphNode(&node, root, nullptr, 0, g);
         cudaGraphDestroy(g);

@@ -157,7 +157,8 @@ static void launch_acu_uv(const AcuArgs& A, cudaStream_t s) {
 // 900 tiles of 100 levels 89.5 / 75.8), so the waves decide (launch_acu_column): 2048 tiles of
 // 80 levels stay at 98.8 us with 12 workers (102.5 with 8).  Measured beside them at 505 /
 // 2048 tiles: 16 workers and two CTAs 20.6 us, 20 and two 26.8 us, 24 and one 32.9 us, 8 and
-// five (40 registers) 20.6 / 157 us, 4 and six 18.6 / 156 us.
+// five (40 registers) 20.6 / 157 us, 4 and six 18.6 / 156 us.  The 12-worker form keeps to 48
+// registers with spills of 64 B of stores and 100 B of loads a thread; the 8-worker form has none.
 constexpr int kColTile = 32;
 constexpr int kEpiChunk = 7;  // epilogue levels per worker per chunk (5: 102 us, 10: 112 us at 2048 tiles, 8 workers)
 template <int LEVELS>
@@ -845,7 +846,8 @@ __global__ void __launch_bounds__(kAdvTX* kAdvTY, AdvMinBlocks<KIND>::value) k_a
 // -> 111 / 104 us, 640x512x20 105 / 101 -> 80 / 75 us, 192x192x64 (2688 warps) 39 / 35 -> 37 /
 // 33 us; 128x128x64 (1280 warps) 18.6 -> 26 us, so from 16 warps an SM.  Measured beside it at
 // 256x256x80: 1 row a thread 77 / 72 us, 3 rows 78 / 69, 4 rows (spilling) 112 / 84; the
-// staggered and WENO kinds in this form no faster than k_adv_fused.
+// staggered and WENO kinds in this form no faster than k_adv_fused.  80 registers, with 4 B of
+// spills (open edges: 56 B stores, 68 B loads).
 constexpr int kLinRows = 2, kLinX = 31, kLinWarps = 4, kLinLevels = 16;
 
 __device__ __forceinline__ float lin_flux(float m, float v0, float v1, float v2, float v3, float v4, float v5) {

@@ -2388,7 +2388,8 @@ TE_LAUNCH3(morr_prep)
 // walking 40 levels of pow and exp evaluations, and was bound by one warp's latency.  One B200,
 // per launch, thread per column -> this, after 2 / 60 / 140 steps of the recorded storms:
 // 120x120x40 127 / 600 / 961 -> 66 / 104 / 149 us, 300x60x40 132 / 784 / 1214 -> 69 / 162 /
-// 221 us.  8 warps a block 55 / 127 / 177 us, 4 warps 56 / 197 / 283 us on the first.
+// 221 us.  8 warps a block 55 / 127 / 177 us, 4 warps 56 / 197 / 283 us on the first.  16 warps
+// leave 128 registers a thread, 132 B of spill stores and 144 B of loads, and one block an SM.
 //
 // The dispatch's rows are taken scr_rows at a time (the reference's y tiles: the planned
 // per-thread scratch holds that many rows); each launch lays the scratch out by array,

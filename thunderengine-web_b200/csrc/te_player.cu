@@ -930,12 +930,14 @@ cudaGraph_t Plan::capture_step(bool concurrent) {
   return graph;
 }
 
-// The concurrent graph takes 6 (113 nodes) to 25 us (734 nodes) per launch of the step to
-// instantiate, the chain 2-3 us: 2.4 ms for a fused step, 6 ms for the exact one, 17 ms for a
-// recorded full-physics step, which 25 to 35 steps win back.  So the first steps after a
+// Capture and instantiation of the concurrent graph against the chain's, and what a step gains, on
+// one B200 (ms; us a step, chain / concurrent): 107 nodes (fused) 2.3 / 0.36, 12x10x8 271 / 193,
+// 37x29x13 304 / 223, 64x64x40 410 / 352, 128x128x64 1124 / 1038; 130 nodes (exact) 2.9 / 0.47,
+// 322 / 230 (37x29x13), 436 / 368, 1188 / 1093; recorded physics of 602-611 nodes 10 / 1.8,
+// 2787 / 2361 and 3184 / 2774.  So 19 to 36 steps win it back.  The first steps after a
 // change of the step, its parameters, the mode or the stream run as a chain (an adaptive run
-// changes its parameters every step and stays there) and the concurrent graph is
-// built when the same step is launched for the 33rd time.
+// changes its parameters every step and stays there), and the call that launches the same
+// step for the 33rd time builds the concurrent graph.
 constexpr int kChainRuns = 32;
 
 void Plan::launch_step_graph() {
