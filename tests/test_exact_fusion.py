@@ -208,3 +208,37 @@ def test_a_store_on_closed_edges_is_not_repeated_on_open_ones():
     for stage, opened in ((0, False), (1, True)):
         _adv_u(tape, run, stage, opened, copy.deepcopy(rk))
     _same_words(run, tape, run.initial_buffers(), 0)
+
+
+# Fields in a buffer that is not marked as an arena; acoustic_pp's binding 9 left at an earlier
+# kernel's field (w) in the substeps that store nothing there: all substeps fuse in fused mode
+@pytest.mark.gpu
+@pytest.mark.parametrize('form', ['no arena', 'no ppx'])
+def test_forms_that_stay_fused(form):
+    run = _run()
+    tape = run.tape(1)
+    if form == 'no arena':
+        for b in tape['buffers']:
+            b['arena'] = False
+    else:
+        cmds, held = [], []
+        for c in tape['steps'][0]:   # binding 9 of acoustic_pp where it does not store there
+            if c['op'] == 'pipe':
+                held = [c] if c['name'] == 'acoustic_pp' else []
+            if not held:
+                cmds.append(c)
+                continue
+            if c is not held[0]:
+                held.append(c)
+            if c['op'] == 'dispatch':
+                save = next(h for h in held if h['op'] == 'bytes' and h['index'] == 10)
+                if struct.unpack('<i', base64.b64decode(save['data'])[:4])[0] == 0:
+                    held = [h for h in held if not (h['op'] == 'buf' and h['index'] == 9)]
+                cmds += held
+                held = []
+        tape['steps'][0] = cmds
+    r = helpers.gpu_replayer(tape, {}, hashes=False, mode=1)
+    assert sum(s[0] == 1 for s in r.fused_segments()) == 11
+    r.close()
+    for mode in (0, 1):
+        _same_words(run, tape, run.initial_buffers(), mode)

@@ -1340,14 +1340,18 @@ static bool match_substep(const std::vector<Op>& ops, size_t i, FusedSegment& s,
   return true;
 }
 
-// No field written is read or written twice, and none overlaps another.
-static bool separate_fields(const Plan& P, const std::vector<const float*>& wr, const std::vector<const float*>& rd) {
+// No field written is read or written twice, and none overlaps another (a field of grid g, which is
+// all of its region that the phases' kernels touch).
+static bool separate_fields(const Plan& P, const Dims& g, const std::vector<const float*>& wr,
+                            const std::vector<const float*>& rd) {
+  const uint64_t bytes = (uint64_t)g.sJ * g.sK * ((uint64_t)g.nz + 1) * 4;
   std::vector<Access> all;
   all.reserve(wr.size() + rd.size());
   for (const auto* fields : {&wr, &rd})
     for (const float* f : *fields) {
       if (!f) return false;
       all.push_back(P.access(f, false));
+      all.back().hi = std::min<uint64_t>(all.back().hi, all.back().lo + bytes);
     }
   for (size_t a = 0; a < wr.size(); a++)
     for (size_t b = a + 1; b < all.size(); b++)
@@ -1388,7 +1392,7 @@ static bool match_flux_div(const Plan& P, const std::vector<Op>& ops, size_t i, 
     A.rrw = flux[2];
     A.rho0 = mf.args.p[4];
     A.rf0 = mf.args.p[5];
-    if (!separate_fields(P, {A.rru, A.rrv, A.rrw, A.divx}, {A.u, A.v, A.w, A.rho0, A.rf0, A.mh, A.hm})) return false;
+    if (!separate_fields(P, g, {A.rru, A.rrv, A.rrw, A.divx}, {A.u, A.v, A.w, A.rho0, A.rf0, A.mh, A.hm})) return false;
   } else {
     for (int q = 0; q < 3; q++)
       if (first.args.p[1 + q] != flux[q]) return false;
@@ -1400,8 +1404,8 @@ static bool match_flux_div(const Plan& P, const std::vector<Op>& ops, size_t i, 
     A.rf0 = mf.args.p[2];
     A.mh3 = first.args.p[4];
     A.div3d = first.args.p[5];
-    if (!separate_fields(P, {A.div3d, A.divx}, {A.u, A.v, A.w, A.rho0, A.rf0, A.mh, A.mh3, A.hm})) return false;
-    if (!separate_fields(P, {A.u, A.v, A.w}, {A.rho0, A.rf0, A.mh, A.mh3, A.hm})) return false;
+    if (!separate_fields(P, g, {A.div3d, A.divx}, {A.u, A.v, A.w, A.rho0, A.rf0, A.mh, A.mh3, A.hm})) return false;
+    if (!separate_fields(P, g, {A.u, A.v, A.w}, {A.rho0, A.rf0, A.mh, A.mh3, A.hm})) return false;
   }
   s.kind = kFluxDiv;
   s.first = (int)i;
@@ -1596,7 +1600,8 @@ static bool plain_bindings(const Plan& P, const std::vector<Op>& ops, const Fuse
   if (s.kind == kAcoustic) {
     const AcuArgs& A = D.acu[s.aux[0]];
     const Op &fp = ops[s.first + 1], &ws = ops[s.first + 2];
-    wr = {A.ppd, A.u, A.v, A.w, A.rru, A.rrv, A.rrw, A.pp3d, A.ppx, fp.args.p[11], ws.args.p[10], ws.args.p[11]};
+    wr = {A.ppd, A.u, A.v, A.w, A.rru, A.rrv, A.rrw, A.pp3d, fp.args.p[11], ws.args.p[10], ws.args.p[11]};
+    if (A.saveX) wr.push_back(A.ppx);
     rd = {A.thv, A.uten, A.vten, A.hm, A.piadv, A.ppten, A.ppterm, A.pk1, A.pk2, A.qk, A.mm, A.wten};
   } else if (s.kind == kAdvect) {
     const AdvArgs& A = D.adv[s.aux[0]];
@@ -1610,7 +1615,7 @@ static bool plain_bindings(const Plan& P, const std::vector<Op>& ops, const Fuse
   } else {
     return true;  // kFluxDiv: match_flux_div
   }
-  return separate_fields(P, wr, rd);
+  return separate_fields(P, ops[s.first].args.g, wr, rd);
 }
 
 // keep_scratch (exact mode): a phase stays fused when every store it skips is made again later in
