@@ -34,3 +34,35 @@ def test_gradient_and_memory_of_repeated_windows(dims, steps, every):
     for q in grads[1:]:
         for a, b in zip(q, grads[0]):
             assert np.linalg.norm(a - b) <= 1e-5 * np.linalg.norm(b)
+
+
+# A new time step (use_step, the same structure) between windows: tables and graphs follow it
+@pytest.mark.gpu
+def test_gradient_after_a_change_of_parameters():
+    run = timestep.Run(scenario.tiny(16, 12, 6, dx=500.0, dz=250.0, dt=3.0, nsound=7, us=25.0), core=True)
+    tape = run.tape(1)
+    start = helpers.cpu_run(tape, run.initial_buffers(), nsteps=1, hashes=False)
+    init = {b['id']: start.buffer_words(b['id']).tobytes() for b in tape['buffers']}
+    core = run.tape(1, core=True)
+    run.set_time_step(2.0, 7)
+    later = run.tape(1, core=True)
+    seed = np.random.default_rng(5).standard_normal(run.grid.count).astype(np.float32)
+
+    def gradient(r):
+        base = r.base[run.rec.ids['arena']]
+        r.adjoint_forward(4, 2)
+        r.adjoint_write_words(base + run.fields['w'] // 4, seed)
+        r.adjoint_backward()
+        return [r.adjoint_read(run.grid.count, base + run.fields[n] // 4).astype(np.float64) for n in ('th', 'u_a', 'v_a')]
+
+    fresh = helpers.gpu_replayer(later, init, hashes=False)
+    want = gradient(fresh)
+    fresh.close()
+    r = helpers.gpu_replayer(core, init, hashes=False)
+    other = gradient(r)
+    r.use_step(later['steps'][0])
+    got = [gradient(r) for _ in range(5)][-1]   # 20 steps: past the chain
+    r.close()
+    for a, b, c in zip(got, want, other):
+        assert np.linalg.norm(a - b) <= 1e-5 * np.linalg.norm(b)
+        assert np.linalg.norm(c - b) > 1e-3 * np.linalg.norm(b)

@@ -421,7 +421,8 @@ struct AdjointState {
   std::vector<uint32_t*> ckpt;
   uint64_t ckpt_words = 0;
   int nsteps = 0, every = 0;
-  const Step* step = nullptr;  // the step the tables below were built for
+  const Step* step = nullptr;  // the step the tables below were built for, and its arguments
+  unsigned args_version = 0;
   std::vector<std::vector<Region>> regions;  // per op: the regions it writes
   std::vector<adj::AdjArgs<float>> args;     // per op
   std::vector<adj::AdjLaunch> launch;        // per op (nullptr for copies)
@@ -498,7 +499,7 @@ void in_order(StepDeps* deps, const std::vector<Access>& acc, F launch) {
 
 // Per-op tables of the active step: written regions, adjoint arguments and operators.
 void build_tables(Plan& P, AdjointState& S) {
-  if (S.step == P.active && !S.args.empty()) return;
+  if (S.step == P.active && S.args_version == P.args_version && !S.args.empty()) return;
   S.drop_graphs();
   const std::vector<Op>& ops = P.active->ops;
   S.regions.assign(ops.size(), {});
@@ -630,6 +631,7 @@ void build_tables(Plan& P, AdjointState& S) {
     i = e;
   }
   S.step = P.active;
+  S.args_version = P.args_version;
 }
 
 // Saves the regions of one op in the undo log from word `cur` of the step's part on, or restores

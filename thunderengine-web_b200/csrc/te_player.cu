@@ -396,6 +396,7 @@ void Plan::finalize_args(std::vector<Op>& ops) {
   }
   for (size_t i = 0; i < ops.size(); i++)
     if (!ops[i].copy && ops[i].spec && ops[i].bound) ops[i].args = args[i];
+  args_version++;
   struct Bound {
     uint64_t lo, hi;
     bool write;

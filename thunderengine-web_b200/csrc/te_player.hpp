@@ -77,6 +77,7 @@ struct Plan {
   std::map<std::string, KMeta> kmeta;
   std::map<std::string, Step> cache;
   Step* active = nullptr;
+  unsigned args_version = 0;     // changes with the arguments of any step
   std::vector<KArgs> new_args;  // finalize_args: arguments until all of them are checked
   std::vector<Op> diag_ops;
   // device
