@@ -493,12 +493,11 @@ int te_plan(te_ctx* ctx, const char* tape_json, size_t tape_len, const char* ker
   const uint64_t bytes = P.mem_words * 4, more = te::FusedStep::chains_substeps(P.active->ops) ? 2 * P.field_stride : 0;
   if (more && cudaMalloc(&P.M, bytes + more) == cudaSuccess) {
     P.work = reinterpret_cast<float*>(P.M + P.mem_words);
-    CU(cudaMemsetAsync(P.work, 0, more, ctx->plan.stream));
   } else {
     cudaGetLastError();
     CU(cudaMalloc(&P.M, bytes));
   }
-  CU(cudaMemsetAsync(P.M, 0, P.mem_words * 4, ctx->plan.stream));
+  CU(cudaMemsetAsync(P.M, 0, bytes + (P.work ? more : 0), ctx->plan.stream));
   CU(cudaMalloc(&P.H, std::max<size_t>(16, (size_t)P.hash_count * 4)));
   CU(cudaMemsetAsync(P.H, 0, std::max<size_t>(16, (size_t)P.hash_count * 4), ctx->plan.stream));
   for (auto& bi : P.bytes_init)
